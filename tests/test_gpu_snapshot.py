@@ -59,3 +59,25 @@ def test_sph_snapshot_replays_bit_for_bit(gpu, prec):
     b = g.getSPH()
     for k in ("position", "velocity", "density", "pressure", "densityChange"):
         np.testing.assert_array_equal(a[k], b[k])
+
+
+@pytest.mark.parametrize("steps", [(), (5,)])
+def test_sph_snapshot_keeps_a_pending_rebuild(gpu, steps):
+    """A snapshot taken while the skin rows wait for their rebuild (none was
+    built yet, or the lists were just resized) restores with the rebuild still
+    pending: the steps after it repeat exactly, twice."""
+    sc = scenes.dam_break_reference()
+    g = build_sph(sc, "fp64")
+    for n in steps:
+        g.step(n)
+        g.synchronize()
+    snap = g.snapshot()
+    g.step(20)
+    a = g.getSPH()
+    assert np.abs(a["pressure"]).max() > 0
+    for _ in range(2):
+        snap.restore()
+        g.step(20)
+        b = g.getSPH()
+        for k in ("position", "velocity", "density"):
+            np.testing.assert_array_equal(a[k], b[k])

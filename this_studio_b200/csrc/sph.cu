@@ -2458,7 +2458,7 @@ struct SphScene {
     // Saved dynamic state for overflow replay.
     struct Snap {
         std::vector<std::unique_ptr<DBuf<char>>> bufs;
-        std::vector<void*> dst;
+        std::vector<void*> dst;  // the scene's DBuf objects (a regrowth may move their memory)
         std::vector<size_t> bytes;
         long iStep;
         double time;
@@ -2467,6 +2467,7 @@ struct SphScene {
         // that the steps after a restore use the rows the steps after the
         // snapshot used; valid while the list capacities are unchanged
         bool lists = false;
+        size_t skin = 0;  // index of the copied rebuild state
         int KF = 0, KD = 0;
         bool haveLists = false;
     };
@@ -2479,7 +2480,7 @@ struct SphScene {
         auto c = std::make_unique<DBuf<char>>();
         c->alloc(b.bytes(), s, false);
         snapCopies.push_back({c->p, b.p, b.bytes()});
-        sn.dst.push_back((void*)b.p);
+        sn.dst.push_back((void*)&b);
         sn.bytes.push_back(b.bytes());
         sn.bufs.push_back(std::move(c));
     }
@@ -2497,6 +2498,7 @@ struct SphScene {
         if (sn.lists) {
             sn.KF = KF; sn.KD = KD; sn.haveLists = haveLists;
             snap_add(sn, nbV); snap_add(sn, cntV); snap_add(sn, nbVD); snap_add(sn, cntVD); snap_add(sn, xb);
+            sn.skin = sn.bufs.size();
             snap_add(sn, skinState);
             snap_add(sn, posf);
         }
@@ -2506,15 +2508,17 @@ struct SphScene {
         snapCopies.clear();
         for (size_t k = 0; k < sn.bufs.size(); k++) {
             if (!lists && k >= 6) break;  // the state records come first
-            snapCopies.push_back({sn.dst[k], sn.bufs[k]->p, sn.bytes[k]});
+            snapCopies.push_back({((DBuf<char>*)sn.dst[k])->p, sn.bufs[k]->p, sn.bytes[k]});
         }
         g_launches += copy_list(snapCopies, s);
         DEMSPH_LAUNCH_CHECK();
         iStep = sn.iStep; time = sn.time; P = sn.P; Vv = sn.Vv; S = sn.S; R0 = sn.R0; D = sn.D; ID = sn.ID; L = sn.L;
         refresh_shadows();  // the FP32 / fixed-point copies follow the restored records (and force a skin rebuild)
         if (lists) {
-            // the restored rows and rebuild state stand: no forced rebuild
-            DEMSPH_CUDA(cudaMemsetAsync(&skinState.p->force, 0, 1, s));
+            // the restored rows and rebuild state stand, a rebuild that was
+            // pending at the snapshot (its rows are not the state's) included
+            DEMSPH_CUDA(cudaMemcpyAsync(&skinState.p->force, sn.bufs[sn.skin]->p + offsetof(SkinState, force),
+                                        sizeof(int), cudaMemcpyDeviceToDevice, s));
             haveLists = sn.haveLists;
         }
     }
