@@ -1,0 +1,109 @@
+"""The pair-parallel force evaluation and the list build at the sizes where
+their forms change: crowded stencil rows (more candidates than a row's mask
+holds), rows that outgrow their capacity, scenes on either side of the list
+build's and the finish's lane limits, walls whose balls touch few or many
+triangles, and springs that end with their contact.  Against the FP64 oracle;
+FP64 sums in another order differ by their rounding (1e-11 relative leaves a
+factor 1000 over the 1e-14 of an evaluation for the steps to amplify it)."""
+import numpy as np
+import pytest
+
+from this_studio_b200 import scenes
+from this_studio_b200.scenes import DEMScene, build_dem, hertz_params
+
+from .helpers import oracle_dem, pair_keys, rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+def _crowd(n_small, n_big, seed=4):
+    """A few large balls (first, so that they point at everything near) among
+    many small ones: cells as wide as the large balls hold dozens of candidates."""
+    rng = np.random.default_rng(seed)
+    L = 0.1 * (n_small / 1500.0) ** (1.0 / 3.0)
+    pos = rng.uniform(0, L, (n_big + n_small, 3))
+    rad = np.r_[np.full(n_big, 0.012), rng.uniform(0.0012, 0.002, n_small)]
+    Es, Gs = hertz_params(1e6, 0.3)
+    sc = DEMScene(name="crowd", position=pos, radius=rad, density=np.full(len(rad), 2500.0),
+                  material=np.zeros(len(rad), np.int32), velocity=rng.normal(0, 0.05, pos.shape),
+                  hertz=[(0, 0, Es, Gs, 0.8, 0.2, 0.1, 0.3, 0.05, 0.05)], minb=(-0.03,) * 3, maxb=(L + 0.03,) * 3,
+                  dt=1e-6)
+    return sc
+
+
+def _compare(sc, steps, prec="fp64", tol=1e-11):
+    g, o = build_dem(sc, prec), oracle_dem(sc)
+    if getattr(sc, "constant_force", None) is not None:
+        o.set_constant_force(sc.constant_force)
+    for n in steps:
+        g.step(n)
+        o.step(n)
+        p, q = g.getPairs(0), o.pairs(0)
+        np.testing.assert_array_equal(pair_keys(p["objectPointed"], p["objectPointing"]), pair_keys(q["a"], q["b"]))
+        b, c = g.getBall(), o.balls()
+        for k, r in (("position", "pos"), ("velocity", "vel"), ("angularVelocity", "angvel"), ("force", "force")):
+            assert rel_err(b[k], c[r]) < tol, (n, k)
+    return g, o
+
+
+@pytest.mark.parametrize("n_small,n_big", [(1500, 6), (20000, 40)])
+def test_crowded_rows_and_regrowth(gpu, n_small, n_big):
+    _compare(_crowd(n_small, n_big), (3, 9))
+
+
+@pytest.mark.parametrize("side", [25, 26])  # 15,625 and 17,576: either side of the build's lane limit
+def test_list_build_forms_agree_with_the_oracle(gpu, side):
+    _compare(scenes.dem_pack(n_side=side), (5, 6))
+
+
+@pytest.mark.parametrize("n", [250_000, 275_000])  # 250,047 and 274,625: either side of the finish's lane limit
+def test_finish_forms_agree_with_the_oracle(gpu, n):
+    sc = scenes.dem_drop_poly(n, seed=2)
+    rng = np.random.default_rng(1)
+    sc.position[:, 2] -= 0.1 * 0.005 * np.sqrt(3.0)
+    sc.position[:, :2] *= 0.8  # neighbours in a row touch
+    sc.velocity = rng.normal(0, 0.2, sc.position.shape) + np.array([0, 0, -0.5])
+    _compare(sc, (6,))
+
+
+def test_springs_end_with_their_contact(gpu):
+    """Spheres that touch, slide and part: a pair apart keeps neither its force
+    nor its springs, and a restored state evaluates afresh."""
+    sc = scenes.dem_pack(n_side=5, overlap=0.002, vel=0.6)
+    g, o = _compare(sc, (1, 7, 12, 30))
+    p, q = g.getPairs(0), o.pairs(0)
+    apart = np.linalg.norm(p["force"], axis=1) == 0
+    assert apart.any() and not apart.all()
+    assert np.abs(p["sliding"][apart]).max() == 0 and np.abs(p["torqueB"][apart]).max() == 0
+    snap = g.snapshot()
+    g.step(13)
+    a = g.getBall()
+    snap.restore()
+    g.step(13)
+    for k, v in g.getBall().items():
+        np.testing.assert_array_equal(v, a[k])
+
+
+@pytest.mark.parametrize("segments", [(4, 1), (10, 3), (40, 40)])  # 16 triangles with the caps, 80, 3,280
+def test_walls_of_few_and_many_triangles(gpu, segments):
+    """Balls pressed onto a capped cylinder: up to dozens of candidate
+    triangles per ball on the fine mesh, a handful on the coarse ones."""
+    rng = np.random.default_rng(9)
+    mesh = scenes.cylinder_mesh((0.0, 0.0, 0.0), (0.0, 0.0, 1.0), 0.05, 0.08, *segments)
+    r = 0.006
+    t = rng.uniform(0, 2 * np.pi, 120)
+    pos = np.stack([(0.05 + 0.9 * r) * np.cos(t), (0.05 + 0.9 * r) * np.sin(t), rng.uniform(-0.03, 0.03, 120)], 1)
+    keep = [0]
+    for k in range(1, len(pos)):
+        if np.linalg.norm(pos[keep] - pos[k], axis=1).min() > 2.0 * r:
+            keep.append(k)
+    pos = pos[keep]
+    Es, Gs = hertz_params(1e7, 0.3)
+    sc = DEMScene(name="cyl", position=pos, radius=np.full(len(pos), r), density=np.full(len(pos), 2500.0),
+                  material=np.zeros(len(pos), np.int32), velocity=rng.normal(0, 0.1, pos.shape) - 2.0 * pos,
+                  hertz=[(0, 0, Es, Gs, 0.8, 0.2, 0.1, 0.3, 0.05, 0.05)],
+                  walls=[dict(mesh, position=(0.0, 0.0, 0.0), material=0)], minb=(-0.1,) * 3, maxb=(0.1,) * 3, dt=5e-6)
+    g, o = _compare(sc, (1, 10), tol=1e-10)
+    p, q = g.getPairs(1), o.pairs(1)
+    np.testing.assert_array_equal(pair_keys(p["objectPointed"], p["objectPointing"]), pair_keys(q["a"], q["b"]))
+    assert len(p["objectPointed"]) > 0

@@ -19,6 +19,10 @@ struct MatPair {
     double kn, ks, kr, kt, dn, ds, dr, dt;
     // Hertz-Mindlin (contactParameters.h:62-73)
     double E, G, D, krks, ktks;
+    // damping per sqrt(m sqrt(R delta)): 2 sqrt(5/6) D sqrt(k / sqrt(R delta)) for
+    // the normal, sliding, rolling and torsion stiffnesses, all of which grow as
+    // sqrt(R delta) (one square root per contact instead of five)
+    double zn, zs, zr, zt;
     // friction (the active model's)
     double mus, mur, mut;
     // parallel bond (contactParameters.h:91-100)
@@ -37,45 +41,47 @@ __host__ __device__ __forceinline__ int pair_param_index(int a, int b, int nMat,
 }
 
 // --------------------------------------------------------------- springs ---
-// integrateSlidingOrRollingSpring (contactKernel.cuh:64-97).  The spring is
-// accumulated in FP64; the trial force for the Coulomb cap uses R.
+// The Coulomb cap: the spring s unless its trial force -(k s) - c v exceeds
+// mu |Fn|, else the spring whose force lies on the cap.  In FP64 the squares are
+// compared (a square root only for a capped spring); in FP32 the lengths, whose
+// squares could underflow.
 template <class R>
-__host__ __device__ __forceinline__ double3 spring_slide(double3 sp, V<R> sv, double3 n, V<R> Fn, R mu, R k, R c, double dt) {
-    double3 s = mk3(0, 0, 0);
-    if (k > (R)0) {
-        double3 s1 = sp - dot(sp, n) * n;
-        double a1 = len(s1);
-        if (a1 > 1.e-10) s1 *= len(sp) / a1;
-        s = s1 + up(sv) * dt;
-        if (mu > (R)0) {
-            V<R> fs = -(cvt<R>(s) * k) - sv * c;
-            R af = rlen(fs), an = rlen(Fn);
-            if (af > mu * an) {
-                R ratio = mu * an / af;
-                fs = fs * ratio;
-                s = -(up(fs) + up(sv * c)) / (double)k;
-            }
+__host__ __device__ __forceinline__ double3 spring_cap(double3 s, V<R> v, V<R> Fn, R mu, R k, R c) {
+    if (mu > (R)0) {
+        V<R> fs = -(cvt<R>(s) * k) - v * c;
+        bool over;
+        R ratio = (R)1;
+        if constexpr (sizeof(R) == 8) {
+            const R af2 = dot(fs, fs), cap2 = mu * mu * dot(Fn, Fn);
+            over = af2 > cap2;
+            if (over) ratio = rsq(cap2 / af2);
+        } else {
+            const R af = rlen(fs), an = rlen(Fn);
+            over = af > mu * an;
+            if (over) ratio = mu * an / af;
+        }
+        if (over) {
+            fs = fs * ratio;
+            s = -(up(fs) + up(v * c)) / (double)k;
         }
     }
     return s;
 }
+// integrateSlidingOrRollingSpring (contactKernel.cuh:64-97).  The spring is
+// accumulated in FP64; the trial force for the Coulomb cap uses R.
+template <class R>
+__host__ __device__ __forceinline__ double3 spring_slide(double3 sp, V<R> sv, double3 n, V<R> Fn, R mu, R k, R c, double dt) {
+    if (!(k > (R)0)) return mk3(0, 0, 0);
+    double3 s1 = sp - dot(sp, n) * n;
+    const double a2 = len2(s1);
+    if (a2 > 1.e-20) s1 *= sqrt(len2(sp) / a2);
+    return spring_cap<R>(s1 + up(sv) * dt, sv, Fn, mu, k, c);
+}
 // integrateTorsionSpring (contactKernel.cuh:99-126)
 template <class R>
 __host__ __device__ __forceinline__ double3 spring_torsion(double3 sp, V<R> tv, double3 n, V<R> Fn, R mu, R k, R c, double dt) {
-    double3 s = mk3(0, 0, 0);
-    if (k > (R)0) {
-        s = dot(sp + up(tv) * dt, n) * n;
-        if (mu > (R)0) {
-            V<R> fs = -(cvt<R>(s) * k) - tv * c;
-            R af = rlen(fs), an = rlen(Fn);
-            if (af > mu * an) {
-                R ratio = mu * an / af;
-                fs = fs * ratio;
-                s = -(up(fs) + up(tv * c)) / (double)k;
-            }
-        }
-    }
-    return s;
+    if (!(k > (R)0)) return mk3(0, 0, 0);
+    return spring_cap<R>(dot(sp + up(tv) * dt, n) * n, tv, Fn, mu, k, c);
 }
 
 // LinearContact / HertzianMindlinContact (contactKernel.cuh:128-290) after
@@ -138,13 +144,9 @@ __host__ __device__ __forceinline__ void contact_law(const MatPair& mp, V<R>& F,
         R sq = rsq((R)Rad * (R)delta);
         R kn = (R)(4. / 3.) * (R)mp.E * sq;
         R ks = (R)8 * (R)mp.G * sq;
-        R s56 = rsq((R)(5. / 6.));
-        R mr = (R)m, D = (R)mp.D;
-        R cn = (R)2 * s56 * D * rsq(mr * kn);
-        R cs = (R)2 * s56 * D * rsq(mr * ks);
         R kr = ks * (R)mp.krks, kt = ks * (R)mp.ktks;
-        R cr = (R)2 * s56 * D * rsq(mr * kr);
-        R ct = (R)2 * s56 * D * rsq(mr * kt);
+        R sm = rsq((R)m * sq);
+        R cn = (R)mp.zn * sm, cs = (R)mp.zs * sm, cr = (R)mp.zr * sm, ct = (R)mp.zt * sm;
         law_tail<R>(F, T, es, er, et, vc, wij, n, (R)delta, (R)Rad, dt, kn, ks, kr, kt, cn, cs, cr, ct, (R)mp.mus,
                     (R)mp.mur, (R)mp.mut, roll, tors);
     }
