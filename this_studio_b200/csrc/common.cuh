@@ -359,6 +359,102 @@ struct DBuf {
 
 static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
 
+// (x, y, z) of n records as packed doubles.
+static __global__ void k_take3(size_t n, const double4* __restrict__ src, double* __restrict__ dst) {
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const double4 a = src[t];
+    dst[3 * t] = a.x;
+    dst[3 * t + 1] = a.y;
+    dst[3 * t + 2] = a.z;
+}
+// A getter's device records into the caller's arrays: vectors packed on the
+// device, then everything through two halves of the page-locked staging, one
+// half on the link while host threads empty the other (a pageable copy of whole
+// records and a serial repacking loop took 38 of a 1M-sphere read-back's 40 ms).
+class Readback {
+  public:
+    void vec3(double* host, const double4* src, size_t n) {
+        if (host && n) items_.push_back({(char*)host, (const char*)src, n * 3 * sizeof(double), true});
+    }
+    void raw(void* host, const void* src, size_t bytes) {
+        if (host && bytes) items_.push_back({(char*)host, (const char*)src, bytes, false});
+    }
+    // Returns the kernels launched; the caller's arrays are filled on return.
+    int run(cudaStream_t s) {
+        int launches = 0;
+        size_t words = 0;
+        for (const Item& it : items_)
+            if (it.take3) words += it.bytes / sizeof(double);
+        DBuf<double> packed;
+        packed.alloc(words, s, false);
+        double* q = packed.p;
+        for (Item& it : items_) {
+            if (!it.take3) continue;
+            const size_t n = it.bytes / (3 * sizeof(double));
+            k_take3<<<grid_for(n, 256), 256, 0, s>>>(n, (const double4*)it.src, q);
+            launches++;
+            it.src = (const char*)q;
+            q += 3 * n;
+        }
+        DEMSPH_LAUNCH_CHECK();
+        PinnedStage& ps = PinnedStage::get();
+        std::lock_guard<std::mutex> lk(ps.m);
+        char* st = ps.reserve(2 * kHalf);
+        if (!st) {  // no page-locked memory: straight into the caller's arrays
+            for (const Item& it : items_)
+                DEMSPH_CUDA(cudaMemcpyAsync(it.host, it.src, it.bytes, cudaMemcpyDeviceToHost, s));
+            DEMSPH_CUDA(cudaStreamSynchronize(s));
+            return launches;
+        }
+        // pieces of at most kHalf bytes, several small items to a half
+        struct Half {
+            std::vector<Item> part;
+            cudaEvent_t ev = nullptr;
+            ~Half() {
+                if (ev) cudaEventDestroy(ev);
+            }
+        } half[2];
+        for (Half& h : half) DEMSPH_CUDA(cudaEventCreateWithFlags(&h.ev, cudaEventDisableTiming));
+        size_t k = 0, off = 0;
+        auto fill = [&](int h) {
+            half[h].part.clear();
+            size_t used = 0;
+            while (k < items_.size() && used < kHalf) {
+                const Item& it = items_[k];
+                const size_t len = std::min(it.bytes - off, kHalf - used);
+                DEMSPH_CUDA(cudaMemcpyAsync(st + h * kHalf + used, it.src + off, len, cudaMemcpyDeviceToHost, s));
+                half[h].part.push_back({it.host + off, st + h * kHalf + used, len, false});
+                used += len;
+                off += len;
+                if (off == it.bytes) {
+                    k++;
+                    off = 0;
+                }
+            }
+            DEMSPH_CUDA(cudaEventRecord(half[h].ev, s));
+        };
+        fill(0);
+        for (int h = 0; !half[h].part.empty(); h ^= 1) {
+            fill(h ^ 1);
+            DEMSPH_CUDA(cudaEventSynchronize(half[h].ev));
+            for (const Item& p : half[h].part) host_copy(p.host, p.src, p.bytes);
+        }
+        DEMSPH_CUDA(cudaStreamSynchronize(s));
+        return launches;
+    }
+
+  private:
+    static constexpr size_t kHalf = (size_t)16 << 20;
+    struct Item {
+        char* host;
+        const char* src;
+        size_t bytes;
+        bool take3;
+    };
+    std::vector<Item> items_;
+};
+
 // Chained launches (programmatic dependent launch): a kernel launched with
 // launch_chained may be scheduled while the kernel before it on the stream
 // is still draining, so its launch and block dispatch overlap that kernel's

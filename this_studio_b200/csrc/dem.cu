@@ -2734,22 +2734,19 @@ int demsph_dem_get_balls(demsph_dem_t h, double* pos, double* vel, double* w, do
             }
             return;
         }
-        std::vector<double4> a;
-        auto get = [&](DBuf<double4>& b, double* o) {
-            if (!o) return;
-            b.download(a, s.s);
-            DEMSPH_CUDA(cudaStreamSynchronize(s.s));
-            for (int i = 0; i < s.N(); i++) st3(o, i, xyz(a[i]));
-        };
-        get(s.pos, pos); get(s.vel, vel); get(s.angv, w);
+        const size_t n = (size_t)s.N();
+        Readback rb;
+        rb.vec3(pos, s.pos.p, n);
+        rb.vec3(vel, s.vel.p, n);
+        rb.vec3(w, s.angv.p, n);
         if (s.ready) {
-            get(s.force, force); get(s.torque, torque);
+            rb.vec3(force, s.force.p, n);
+            rb.vec3(torque, s.torque.p, n);
         } else {
-            for (int i = 0; i < s.N(); i++) {
-                if (force) st3(force, i, mk3(0, 0, 0));
-                if (torque) st3(torque, i, mk3(0, 0, 0));
-            }
+            if (force) std::fill(force, force + 3 * n, 0.0);
+            if (torque) std::fill(torque, torque + 3 * n, 0.0);
         }
+        s.launch_count(rb.run(s.s));
     });
 }
 int demsph_dem_set_balls(demsph_dem_t h, const double* pos, const double* vel, const double* w) {
@@ -3012,22 +3009,18 @@ int demsph_dem_get_bonds(demsph_dem_t h, int* a, int* b, int* ok, double* fn, do
         DemScene& s = h->sc;
         int nb = (int)s.hBab.size();
         if (!s.ready) throw Status(DEMSPH_ERR_NOT_READY, "scene not initialised");
-        std::vector<int> OK;
-        std::vector<double> FN, TT;
-        std::vector<double4> FS, TB, NO, PO;
-        s.bok.download(OK, s.s); s.bFn.download(FN, s.s); s.bTt.download(TT, s.s); s.bFs.download(FS, s.s);
-        s.bTb.download(TB, s.s); s.bnormal.download(NO, s.s); s.bpoint.download(PO, s.s);
-        DEMSPH_CUDA(cudaStreamSynchronize(s.s));
+        Readback rb;
+        rb.raw(ok, s.bok.p, nb * sizeof(int));
+        rb.raw(fn, s.bFn.p, nb * sizeof(double));
+        rb.raw(tt, s.bTt.p, nb * sizeof(double));
+        rb.vec3(fs, s.bFs.p, nb);
+        rb.vec3(tb, s.bTb.p, nb);
+        rb.vec3(normal, s.bnormal.p, nb);
+        rb.vec3(point, s.bpoint.p, nb);
+        s.launch_count(rb.run(s.s));
         for (int k = 0; k < nb; k++) {
             if (a) a[k] = s.hBab[k].x;
             if (b) b[k] = s.hBab[k].y;
-            if (ok) ok[k] = OK[k];
-            if (fn) fn[k] = FN[k];
-            if (tt) tt[k] = TT[k];
-            if (fs) st3(fs, k, xyz(FS[k]));
-            if (tb) st3(tb, k, xyz(TB[k]));
-            if (normal) st3(normal, k, xyz(NO[k]));
-            if (point) st3(point, k, xyz(PO[k]));
         }
     });
 }
@@ -3305,15 +3298,13 @@ int demsph_dem_get_clumps(demsph_dem_t h, double* pos, double* vel, double* w, d
         SCENE_CHECK(h);
         DemScene& s = h->sc;
         if (!s.ready) throw Status(DEMSPH_ERR_NOT_READY, "scene not initialised");
-        std::vector<double4> P, Vv, W, Q;
-        s.cpos.download(P, s.s); s.cvel.download(Vv, s.s); s.cangv.download(W, s.s); s.cq.download(Q, s.s);
-        DEMSPH_CUDA(cudaStreamSynchronize(s.s));
-        for (size_t c = 0; c < P.size(); c++) {
-            if (pos) st3(pos, c, xyz(P[c]));
-            if (vel) st3(vel, c, xyz(Vv[c]));
-            if (w) st3(w, c, xyz(W[c]));
-            if (q) { q[4 * c] = Q[c].x; q[4 * c + 1] = Q[c].y; q[4 * c + 2] = Q[c].z; q[4 * c + 3] = Q[c].w; }
-        }
+        const size_t n = s.hCpos.size();
+        Readback rb;
+        rb.vec3(pos, s.cpos.p, n);
+        rb.vec3(vel, s.cvel.p, n);
+        rb.vec3(w, s.cangv.p, n);
+        rb.raw(q, s.cq.p, n * sizeof(double4));
+        s.launch_count(rb.run(s.s));
     });
 }
 int demsph_dem_get_walls(demsph_dem_t h, double* pos, double* q, double* vglobal) {

@@ -316,7 +316,7 @@ class DEMSolver:
 
     def getBall(self):
         n = self.numBalls
-        out = {k: np.zeros((n, 3)) for k in ("position", "velocity", "angularVelocity", "force", "torque")}
+        out = {k: np.empty((n, 3)) for k in ("position", "velocity", "angularVelocity", "force", "torque")}
         call("demsph_dem_get_balls", self._h, _dp(out["position"]), _dp(out["velocity"]),
              _dp(out["angularVelocity"]), _dp(out["force"]), _dp(out["torque"]))
         return out
@@ -398,10 +398,10 @@ class DEMSolver:
 
     def getBondedInteraction(self):
         n = self._n("demsph_dem_num_bonds")
-        out = {"objectPointed": np.zeros(n, np.int32), "objectPointing": np.zeros(n, np.int32),
-               "isBonded": np.zeros(n, np.int32), "normalForce": np.zeros(n), "torsionTorque": np.zeros(n)}
+        out = {"objectPointed": np.empty(n, np.int32), "objectPointing": np.empty(n, np.int32),
+               "isBonded": np.empty(n, np.int32), "normalForce": np.empty(n), "torsionTorque": np.empty(n)}
         for k in ("shearForce", "bendingTorque", "normal", "point"):
-            out[k] = np.zeros((n, 3))
+            out[k] = np.empty((n, 3))
         call("demsph_dem_get_bonds", self._h, _ip(out["objectPointed"]), _ip(out["objectPointing"]),
              _ip(out["isBonded"]), _dp(out["normalForce"]), _dp(out["torsionTorque"]), _dp(out["shearForce"]),
              _dp(out["bendingTorque"]), _dp(out["normal"]), _dp(out["point"]))
