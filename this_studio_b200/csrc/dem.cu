@@ -1413,7 +1413,7 @@ struct DemScene {
         // defaults of buildFromTables (contactKernel.cu:18-31)
         MatPair def{};
         def.linear = 0; def.D = 0.0;  // e = 1 -> ln e = 0
-        def.gamma = 1.0; def.knks = 1.0;
+        def.gamma = 1.0; def.knks = 1.0; def.iknks = 1.0;
         std::vector<MatPair> tab(std::max(cap, 1), def);
         std::vector<double> res(std::max(cap, 1), 1.0);
         for (auto& r : rows.h) {
@@ -1435,7 +1435,7 @@ struct DemScene {
         for (auto& r : rows.bd) {
             int ip = pair_param_index(r.a, r.b, nMat, cap);
             MatPair& m = tab[ip];
-            m.gamma = r.v[0]; m.Eb = r.v[1]; m.knks = r.v[2]; m.sigma = r.v[3]; m.C = r.v[4]; m.mu = r.v[5];
+            m.gamma = r.v[0]; m.Eb = r.v[1]; m.knks = r.v[2]; m.iknks = 1.0 / r.v[2]; m.sigma = r.v[3]; m.C = r.v[4]; m.mu = r.v[5];
         }
         roll = tors = 0;
         for (int ip = 0; ip < (int)tab.size(); ip++) {

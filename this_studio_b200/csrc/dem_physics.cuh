@@ -27,6 +27,7 @@ struct MatPair {
     double mus, mur, mut;
     // parallel bond (contactParameters.h:91-100)
     double gamma, Eb, knks, sigma, C, mu;
+    double iknks;  // 1 / knks
 };
 
 __host__ __device__ __forceinline__ int pair_param_index(int a, int b, int nMat, int cap) {
@@ -152,38 +153,44 @@ __host__ __device__ __forceinline__ void contact_law(const MatPair& mp, V<R>& F,
     }
 }
 
-// Rodrigues rotation (myVec.h:134-176)
-__device__ __forceinline__ double3 rotate_vector(double3 v, double3 ang) {
-    double a2 = dot(ang, ang);
-    if (a2 < 1.0e-20) return v;
-    double a = sqrt(a2);
-    double s, c;
-    sincos(a, &s, &c);
-    double inv = 1.0 / a;
-    double3 k = mk3(ang.x * inv, ang.y * inv, ang.z * inv);
-    double kv = k.x * v.x + k.y * v.y + k.z * v.z;
-    double3 kxv = mk3(k.y * v.z - k.z * v.y, k.z * v.x - k.x * v.z, k.x * v.y - k.y * v.x);
-    double t3 = kv * (1.0 - c);
-    return mk3(v.x * c + kxv.x * s + k.x * t3, v.y * c + kxv.y * s + k.y * t3, v.z * c + kxv.z * s + k.z * t3);
+// Rodrigues rotation (myVec.h:134-176) of two vectors by the rotation vector
+// ang: v cos a + (ang x v) sin a / a + ang (ang . v) (1 - cos a) / a^2.  A bond
+// turns by far less than 0.01 rad per evaluation; there the Taylor series of
+// the three factors in a^2 to a^6 are exact to rounding (the next terms are
+// below 1e-21) and need no square root, division or sincos.
+__device__ __forceinline__ void rotate_two(double3& u, double3& v, double3 ang) {
+    const double a2 = dot(ang, ang);
+    if (a2 < 1.0e-20) return;
+    double c, s, q;  // cos a, sin a / a, (1 - cos a) / a^2
+    if (a2 < 1.0e-4) {
+        s = 1.0 + a2 * (-1.0 / 6.0 + a2 * (1.0 / 120.0 - a2 * (1.0 / 5040.0)));
+        q = 0.5 + a2 * (-1.0 / 24.0 + a2 * (1.0 / 720.0 - a2 * (1.0 / 40320.0)));
+        c = 1.0 - a2 * q;
+    } else {
+        const double a = sqrt(a2);
+        sincos(a, &s, &c);
+        s /= a;
+        q = (1.0 - c) / a2;
+    }
+    u = c * u + s * cross(ang, u) + (q * dot(ang, u)) * ang;
+    v = c * v + s * cross(ang, v) + (q * dot(ang, v)) * ang;
 }
 
 // ParallelBondedContact (contactKernel.cuh:4-62); bond state stays FP64.
 __device__ __forceinline__ int parallel_bond(double& Fn, double& Tt, double3& Fs, double3& Tb, double& smax,
                                              double& tmax, double3 n0, double3 n, double3 vc, double3 wA, double3 wB,
                                              double rA, double rB, double dt, const MatPair& mp) {
-    double3 th1 = cross(n0, n);
-    Fs = rotate_vector(Fs, th1);
-    Tb = rotate_vector(Tb, th1);
-    double3 th2 = dot(0.5 * (wA + wB) * dt, n) * n;
-    Fs = rotate_vector(Fs, th2);
-    Tb = rotate_vector(Tb, th2);
+    rotate_two(Fs, Tb, cross(n0, n));
+    rotate_two(Fs, Tb, dot(0.5 * (wA + wB) * dt, n) * n);
     double rmin = rA < rB ? rA : rB;
     double Rb = mp.gamma * rmin;
     double A = Rb * Rb * kPi;
     double I = Rb * Rb * Rb * Rb / 4. * kPi;
     double J = 2 * I;
+    double iA = 1.0 / A;               // 1 / I = 4 pi / A^2
+    double iI = 4.0 * kPi * iA * iA;
     double knA = mp.Eb / (rA + rB);
-    double ksA = knA / mp.knks;
+    double ksA = knA * mp.iknks;
     double3 dn = dot(vc, n) * n * dt;
     double3 dtr = vc * dt - dn;
     Fn -= dot(dn * knA * A, n);
@@ -193,8 +200,8 @@ __device__ __forceinline__ int parallel_bond(double& Fn, double& Tt, double3& Fs
     double3 rt = wr * dt - rn;
     Tt -= dot(rn * ksA * J, n);
     Tb -= rt * knA * I;
-    smax = -Fn / A + len(Tb) / I * Rb;
-    tmax = len(Fs) / A + fabs(Tt) / J * Rb;
+    smax = -Fn * iA + len(Tb) * iI * Rb;
+    tmax = len(Fs) * iA + fabs(Tt) * (0.5 * iI) * Rb;
     int ok = 1;
     if (mp.sigma > 0 && smax > mp.sigma) ok = 0;
     else if (mp.C > 0 && tmax > mp.C - mp.mu * smax) ok = 0;
