@@ -56,6 +56,40 @@ def test_list_build_forms_agree_with_the_oracle(gpu, side):
     _compare(scenes.dem_pack(n_side=side), (5, 6))
 
 
+@pytest.mark.parametrize("n", [900, 17_000])  # balls: either side of the build's lane limit
+def test_pairs_at_the_cut_off(gpu, n):
+    """Couples of balls at the lists' reach, 1.1 (ra + rb), to within 1e-11 of
+    it and more: an FP32 distance cannot tell these in from out.  The positions
+    are the reference's input, so only the square's FP64 rounding (below 1e-15)
+    separates the two sides, and the nearest couple is 1e-12 from the line.  One
+    larger ball apart widens the cells (twice the largest radius) to the couples'
+    reach, so that no couple lies beyond the stencil."""
+    rng = np.random.default_rng(7)
+    m = n // 2
+    side = int(np.ceil(m ** (1.0 / 3.0)))
+    at = np.stack(np.unravel_index(np.arange(m), (side,) * 3), 1) * 0.08 + 3.0
+    ra, rb = rng.uniform(0.004, 0.01, (2, m))
+    u = rng.normal(size=(m, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    e = 10.0 ** rng.uniform(-12, -4, m) * rng.choice([-1, 1], m)
+    b = at + u * (1.1 * (ra + rb) * (1 + e))[:, None]
+    pos = np.concatenate([at, b, [[2.95] * 3]])
+    rad = np.r_[ra, rb, 0.012]
+    Es, Gs = hertz_params(1e6, 0.3)
+    sc = DEMScene(name="cut-off", position=pos, radius=rad, density=np.full(2 * m + 1, 2500.0),
+                  material=np.zeros(2 * m + 1, np.int32), velocity=np.zeros_like(pos),
+                  hertz=[(0, 0, Es, Gs, 0.8, 0.2, 0.1, 0.3, 0.05, 0.05)], minb=(2.9,) * 3,
+                  maxb=(3.1 + 0.08 * side,) * 3, dt=1e-9)
+    g = build_dem(sc, "fp64")
+    g.step(1)
+    p = g.getPairs(0)
+    d2 = ((at - b) ** 2).sum(1)
+    inside = np.flatnonzero((1.1 * (ra + rb)) ** 2 >= d2)
+    assert 0.4 * m < len(inside) < 0.6 * m
+    ab = np.sort(np.stack([p["objectPointed"], p["objectPointing"]]), axis=0)
+    np.testing.assert_array_equal(np.sort(pair_keys(*ab)), pair_keys(inside, inside + m))
+
+
 @pytest.mark.parametrize("n", [250_000, 275_000])  # 250,047 and 274,625: either side of the finish's lane limit
 def test_finish_forms_agree_with_the_oracle(gpu, n):
     sc = scenes.dem_drop_poly(n, seed=2)

@@ -99,9 +99,12 @@ static __global__ void k_cell_scatter(const int* __restrict__ key, int n, const 
 // itself when orderKey is null): the stable order of the reference sort.  One
 // thread per object counts the cell members that precede it, so a crowded
 // cell costs O(members) per thread instead of a serial insertion sort.
+// rec (or null): the objects' FP32 (x, y, z) from the origin and w, in cell
+// order, so that a stencil row's candidates are one contiguous read.
 static __global__ void k_cell_rank(int n, const int* __restrict__ key, const int* __restrict__ start,
                                    const int* __restrict__ unordered, int* __restrict__ sorted,
-                                   const int* __restrict__ orderKey, int ncell, const int* __restrict__ gate) {
+                                   const int* __restrict__ orderKey, int ncell, const int* __restrict__ gate,
+                                   const double4* __restrict__ p, double3 origin, float4* __restrict__ rec) {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n || (gate && *gate == 0)) return;
     if (s >= start[ncell]) return;  // start[ncell] = objects in the table
@@ -116,6 +119,10 @@ static __global__ void k_cell_rank(int n, const int* __restrict__ key, const int
         r += ku < kv;
     }
     sorted[b + r] = v;
+    if (rec) {
+        const double4 q = p[v];
+        rec[b + r] = make_float4((float)(q.x - origin.x), (float)(q.y - origin.y), (float)(q.z - origin.z), (float)q.w);
+    }
 }
 
 // Host side: owns the cell arrays of one grid and builds them on a stream.
@@ -123,6 +130,7 @@ struct CellTable {
     GridDesc g{};
     int ncell = 0;
     DBuf<int> key, cnt, start, sorted, unordered;
+    DBuf<float4> rec;  // allocated by a user that wants the cell-ordered FP32 records
     std::vector<DBuf<int>*> scanTmp;  // per-level tile sums / offsets
     int launches = 0;                 // kernels issued by the last build
 
@@ -181,7 +189,7 @@ struct CellTable {
         if (n > 0) {
             k_cell_scatter<<<grid_for(n, 256), 256, 0, s>>>(key.p, n, start.p, cnt.p, unordered.p, gate);
             k_cell_rank<<<grid_for(n, 256), 256, 0, s>>>(n, key.p, start.p, unordered.p, sorted.p, orderKey, ncell,
-                                                         gate);
+                                                         gate, p, g.mn, rec.p);
             launches += 2;
         }
         DEMSPH_LAUNCH_CHECK();

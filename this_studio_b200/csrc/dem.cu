@@ -57,6 +57,7 @@ struct DemDev {
     const int* order;      // cell-sorted candidate list (balls, or periodic ghosts)
     const int* qorder;     // the balls that query the lists, in cell order
     const int* cellStart;  // candidate grid
+    const float4* rec;     // the candidates' FP32 (x, y, z) - bg.mn and r, in cell order
     // current / previous pair lists
     int* pj;
     int* pcnt;
@@ -168,10 +169,14 @@ __device__ __forceinline__ void record_pair(const DemDev& d, int slot, int A, in
 // their loops rolled.  kLanes = 8, for small scenes: lane l tests stencil row l
 // (lane 0 the ninth as well) and a prefix over the lanes restores the row
 // order.  kLanes = 1: one thread per ball with the next row's bounds loaded
-// ahead and four candidates in flight.  Against a candidate-by-candidate walk: 4,096
-// touching spheres 40.7 -> 11.5 us (eight lanes; one lane with its loads
-// unrolled took 24.5), 64,000 36.0 -> 26.1 us, 10^6 falling spheres 108 -> 94 us
-// (eight lanes there: 343).
+// ahead and four candidates in flight.  Candidates are read as the sort's
+// cell-ordered FP32 records, 16 contiguous bytes each, where index and FP64
+// position were a gather of 36; the FP64 positions are fetched only for a pair
+// in the test's uncertain band.  Against a candidate-by-candidate walk, and
+// with the gather in between: 4,096 touching spheres 40.7 -> 11.5 -> 10.1 us
+// (eight lanes; one lane with its loads unrolled took 24.5), 64,000
+// 36.0 -> 26.1 -> 25.2 us, 10^6 falling spheres 108 -> 94 -> 84 us (eight lanes
+// there: 343), a beam of 110,000 42 -> 32 us.
 template <int kLanes>
 __global__ void __launch_bounds__(128, kLanes == 1 ? 6 : 8) k_dem_build_pairs(DemDev d) {
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
@@ -193,10 +198,27 @@ __global__ void __launch_bounds__(128, kLanes == 1 ? 6 : 8) k_dem_build_pairs(De
             e = __ldg(d.cellStart + k + st.e.x + 1);
         }
     };
-    auto partner = [&](int B, const double4& pb) {
-        const double cut = 1.1 * (pa.w + pb.w);
-        const double3 r = ra - xyz(pb);
-        if (!((cut * cut - dot(r, r)) >= 0.)) return false;
+    // The distance test on the FP32 records: each coordinate is within 2^-24 of
+    // its magnitude, so |r|^2 is within `band` of the exact one; only inside the
+    // band the FP64 test decides.
+    const float ax = (float)(ra.x - d.bg.mn.x), ay = (float)(ra.y - d.bg.mn.y), az = (float)(ra.z - d.bg.mn.z);
+    const float ar = (float)pa.w, am = fmaxf(fabsf(ax), fmaxf(fabsf(ay), fabsf(az)));
+    auto near = [&](const float4& c, bool& sure) {
+        const float dx = ax - c.x, dy = ay - c.y, dz = az - c.z;
+        const float d2 = dx * dx + dy * dy + dz * dz;
+        const float cut = 1.1f * (ar + c.w), c2 = cut * cut;
+        const float e = 1.2e-7f * (am + cut), band = e * (3.5f * cut + 3.0f * e) + 1.0e-6f * c2;
+        sure = d2 < c2 - band;
+        return d2 <= c2 + band;
+    };
+    auto partner = [&](int B, bool sure) {
+        if (A >= B) return false;
+        if (!sure) {
+            const double4 pb = d.pos[B];
+            const double cut = 1.1 * (pa.w + pb.w);
+            const double3 r = ra - xyz(pb);
+            if (!((cut * cut - dot(r, r)) >= 0.)) return false;
+        }
         // B's mass and clump matter only to a fixed ball and to a pebble
         if (fixedA && d.vel[B].w == 0) return false;
         return !(clA >= 0 && d.clump[B] == clA);
@@ -232,20 +254,22 @@ __global__ void __launch_bounds__(128, kLanes == 1 ? 6 : 8) k_dem_build_pairs(De
             if (row < 8) bounds(row + 1, b1, e1);
 #pragma unroll 1
             for (int k = b; k < e; k += 4) {
-                int B[4];
-                double4 pb[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) B[u] = k + u < e ? __ldg(d.order + k + u) : -1;
+                float4 c[4];
+                unsigned hit = 0, exact = 0;
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    if (A < B[u]) pb[u] = d.pos[B[u]];
-                unsigned hit = 0;
+                    if (k + u < e) c[u] = __ldg(d.rec + k + u);
 #pragma unroll
-                for (int u = 0; u < 4; u++)
-                    if (A < B[u] && partner(B[u], pb[u])) hit |= 1u << u;
+                for (int u = 0; u < 4; u++) {
+                    bool sure = true;
+                    if (k + u < e && near(c[u], sure)) hit |= 1u << u;
+                    if (!sure) exact |= 1u << u;
+                }
                 for (; hit; hit &= hit - 1) {
-                    const int C = d.order[k + __ffs(hit) - 1];
-                    if (total < d.K) keep(C, total);
+                    const int u = __ffs(hit) - 1;
+                    const int B = __ldg(d.order + k + u);
+                    if (!partner(B, !(exact >> u & 1u))) continue;
+                    if (total < d.K) keep(B, total);
                     total++;
                 }
             }
@@ -257,8 +281,8 @@ __global__ void __launch_bounds__(128, kLanes == 1 ? 6 : 8) k_dem_build_pairs(De
         int b[2], e[2], cnt[2];
         unsigned mask[2];  // hits among a row's first 32 candidates
         auto test = [&](int k) {
-            const int B = d.order[k];
-            return A < B && partner(B, d.pos[B]);
+            bool sure;
+            return near(__ldg(d.rec + k), sure) && partner(__ldg(d.order + k), sure);
         };
 #pragma unroll
         for (int q = 0; q < 2; q++) {
@@ -1385,6 +1409,7 @@ struct DemScene {
         d.bincStart = bincStart.p; d.binc = binc.p;
         d.wpos = wpos.p; d.wvel = wvel.p; d.wangv = wangv.p; d.wq = wq.p; d.wmat = wmat.p;
         d.vlocal = vlocal.p; d.vglobal = vglobal.p; d.vwall = vwall.p; d.tris = tris.p; d.tcenter = tcenter.p;
+        d.rec = ballCells.rec.p;
         d.triOrder = triCells.sorted.p; d.triKey = triCells.key.p; d.wmany = wmany.p; d.triCellStart = triCells.start.p; d.wbox = wbox.p;
         int wo = wcur ^ 1;
         d.wtj = wtj[wcur].p; d.wcnt = wcnt[wcur].p; d.wS = wS[wcur].p; d.wR = wR[wcur].p; d.wT = wT[wcur].p;
@@ -1595,6 +1620,7 @@ struct DemScene {
         for (auto& g : ghosts) {
             g->gpos.alloc(N(), s, false);
             g->cells.setup(ballCells.g, N(), s);
+            g->cells.rec.alloc(N(), s, false);
             ghost_alloc(*g);
         }
         gstatus.alloc(1, s, true);
@@ -1629,6 +1655,7 @@ struct DemScene {
         DemDev d = dev(false);
         d.pos = g.gpos.p;
         d.order = g.cells.sorted.p;
+        d.rec = g.cells.rec.p;
         d.cellStart = g.cells.start.p;
         d.K = g.K;
         d.KR = g.KR;
@@ -2054,6 +2081,7 @@ struct DemScene {
         GridDesc bg{};
         if (!grid_set(bg, mn, mx, cell)) throw Status(DEMSPH_ERR_SCENE, "invalid domain or cell size");
         ballCells.setup(bg, n, s);
+        ballCells.rec.alloc(n, s, false);
         double tcell = cell;
         std::vector<double4> cent(hTris.size());
         for (size_t t = 0; t < hTris.size(); t++) {
