@@ -1,0 +1,91 @@
+"""The forms of the fluid passes and of their list build at the sizes and
+states where they change: a single particle, partly filled blocks, either side
+of the sixteen-lane limit, no dummies, particles outside the domain, a domain
+one cell wide, rows that overflow and are walked, exact lists every step.
+The specialised passes against the general ones (FP32: the regrouped terms'
+rounding, 1e-5 as the force target; FP64: sums in another order, 1e-12 over
+the 1e-15 of an evaluation), the pair sets against all pairs within the cutoff."""
+import numpy as np
+import pytest
+
+from this_studio_b200 import scenes
+from this_studio_b200.solvers import WCSPHSolver
+
+from .helpers import pair_keys, rel_err
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"mixed": 1e-5, "fp64": 1e-12}
+
+
+def _scene(nx, ny, nz, dummies=True, seed=1, dx=0.01):
+    sc = scenes.sph_dam_break(nx, ny, nz, dx, tank=(2 * nx * dx, ny * dx, (nz + 2) * dx), column_height=nz * dx)
+    rng = np.random.default_rng(seed)
+    sc.fluid = sc.fluid + rng.uniform(-0.1 * dx, 0.1 * dx, sc.fluid.shape)
+    sc.velocity = rng.normal(0, 0.2, sc.fluid.shape)
+    if not dummies:
+        sc.dummy = np.zeros((0, 3))
+    return sc
+
+
+def _build(sc, prec, uniform=True, skin=None, headroom=None, minb=None, maxb=None):
+    s = WCSPHSolver()
+    if skin is not None:
+        s.setSkin(skin)
+    if headroom is not None:
+        s.setListHeadroom(headroom)
+    s.addSPHs(sc.fluid, sc.velocity, sc.sound_speed, sc.spacing, sc.density, sc.viscosity)
+    if len(sc.dummy):
+        s.addDummies(sc.dummy, None, sc.sound_speed, sc.spacing, sc.density, sc.viscosity)
+    s.initialize(minb or sc.minb, maxb or sc.maxb, sc.gravity, sc.dt, prec)
+    s.setUniformKernels(uniform)
+    return s
+
+
+def _same(a, b, tol):
+    for k in ("velocity", "acceleration", "density", "densityChange"):
+        assert rel_err(a[k], b[k]) < tol or np.abs(a[k] - b[k]).max() < 1e-300, k
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [(1, 1, 1), (3, 2, 2), (5, 7, 9), (20, 20, 20), (21, 20, 20)])  # 8,000 and 8,400 last
+def test_specialised_passes_against_general(gpu, prec, n):
+    sc = _scene(*n)
+    a, b = _build(sc, prec), _build(sc, prec, uniform=False)
+    for steps in (1, 18):
+        a.step(steps)
+        b.step(steps)
+    _same(a.getSPH(), b.getSPH(), TOL[prec])
+    for w in (0, 1):
+        np.testing.assert_array_equal(pair_keys(*a.getPairs(w)), pair_keys(*b.getPairs(w)))
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [(9, 8, 7), (24, 22, 20)])
+def test_no_dummies_and_exact_lists(gpu, prec, n):
+    sc = _scene(*n, dummies=False)
+    ref = _build(sc, prec, uniform=False)
+    free, exact = _build(sc, prec), _build(sc, prec, skin=0.0)
+    for s in (ref, free, exact):
+        s.step(12)
+    _same(free.getSPH(), ref.getSPH(), TOL[prec])
+    _same(exact.getSPH(), ref.getSPH(), TOL[prec])
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [(10, 10, 10), (24, 22, 20)])
+def test_overflowed_rows_are_walked(gpu, prec, n):
+    """No headroom and a compressed start: rows overflow at the first rebuild
+    and the passes walk the cells for them.  After the drift a walked row also
+    takes the pairs that came within the cutoff during it (the listed row does
+    not): a particle moves at most 1e-4 m = 0.004 x 2 h in a step, where the
+    kernel gradient, which falls as the cube of the distance to its edge, is
+    below 1e-6 of its usual size; 1e-5 leaves room for several such pairs."""
+    sc = _scene(*n)
+    a, b = _build(sc, prec, headroom=0.0), _build(sc, prec, uniform=False, headroom=1.0)
+    pos = sc.fluid.copy()
+    pos[:, 2] *= 0.9
+    for s in (a, b):
+        s.setSPH(position=pos)
+        s.step(4)
+    _same(a.getSPH(), b.getSPH(), 1e-5)

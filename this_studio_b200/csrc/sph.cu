@@ -39,19 +39,36 @@ extern std::atomic<long long> g_launches;
 // is needed: grad W = K dq(q_n) r'/|r'| with K = 21 / (16 pi h^4) and
 // q_n = |r'| q / h.
 struct UniK {
-    float invhq;   // q / h
-    float K;       // 21 / (16 pi h^4)
+    // each factor twice, as packed FP32 operands
+    float2 mh;    // -q / (2 h): t = 1 + mh r'
+    float2 fC;    // -5 K q / h: grad W = fC t^3 r'
+    float2 c3;    // 3 (the Riemann limiter's factor)
+    float2 pF, bF;  // fluid pairs: m (pressure, 2 m / 2), 2 nu m (viscosity)
+    float2 pD, bD;  // fluid-dummy pairs: m_dummy, 2 (nu + nu_dummy) / 2 m_dummy
+    float2 dF, dD;  // continuity: 2 / c, 2 / c_bar of the pair
+    // What the FP64 ends of the passes multiply the FP32 sums by: 1 (momentum) or
+    // m / 2 (continuity), with the rounding of the constants above undone.  A
+    // constant's rounding has one sign over all pairs and steps: it would scale
+    // every force and density change alike, a slightly wrong speed of sound.
+    // (aR: the fluid's over the dummies')
+    double aD, aR, sF, sD;
     float c2q;     // (2 h / q)^2, the cutoff in quanta squared
     float cF;      // fluid sound speed
-    float mF2;     // 2 m (fluid)
-    float bF;      // 2 nu m (fluid-fluid viscosity factor)
-    float mF, mD;  // particle masses (continuity)
-    float mD2;     // 2 m_dummy
-    float bD;      // 2 (nu + nu_dummy) / 2 m_dummy
     float cbarD;   // (c + c_dummy) / 2
     float invcD2;  // 1 / c_dummy^2
     float rho0D;   // dummy rest density
     float3 gq;     // gravity times q
+};
+
+// The same constants for the FP64 passes (lengths in metres).
+struct UniD {
+    double cut2;      // (2 h)^2
+    double mh, fC;    // -1 / (2 h), -5 K / h
+    double pF, bF, pD, bD;
+    double dF, dD;
+    double cF, cbarD;
+    double mF, mD;
+    double invcD2, rho0D;
 };
 
 struct SphDev {
@@ -148,6 +165,12 @@ struct SphDev {
     double3 gravity;
     DevStatus* status;
     UniK uk;  // set when the scene qualifies for the specialised passes
+    UniD ud;
+    // the fluid as the specialised FP64 passes gather it: (x, y, z, rho), (v, p)
+    const double4* xr;
+    const double4* vp;
+    double4* xrOut;
+    double4* vpOut;
 };
 
 // A boundary set (dummies or markers) as the fluid passes read it.
@@ -326,7 +349,8 @@ __global__ void k_sph_copy_back(int n, const int* __restrict__ gate, const doubl
                                 double4* __restrict__ pos, double4* __restrict__ vel, double4* __restrict__ st,
                                 double* __restrict__ rho0, double* __restrict__ drho, int* __restrict__ id,
                                 float4* __restrict__ velf, float4* __restrict__ stf, int4* __restrict__ posq,
-                                double4* __restrict__ xb) {
+                                double4* __restrict__ xb, const double4* __restrict__ xr2,
+                                const double4* __restrict__ vp2, double4* __restrict__ xr, double4* __restrict__ vp) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n || *gate == 0) return;
     const double4 p = pos2[t];
@@ -340,6 +364,10 @@ __global__ void k_sph_copy_back(int n, const int* __restrict__ gate, const doubl
     velf[t] = velf2[t];
     stf[t] = stf2[t];
     posq[t] = posq2[t];
+    if (xr) {
+        xr[t] = xr2[t];
+        vp[t] = vp2[t];
+    }
 }
 
 // Skin-list state of a scene, on the device.
@@ -555,7 +583,8 @@ __global__ void k_sph_permute(int n, const int* __restrict__ sorted, const doubl
                               double4* __restrict__ st2, double* __restrict__ rho02, double* __restrict__ drho2,
                               int* __restrict__ id2, float4* __restrict__ posf, float4* __restrict__ velf2,
                               float4* __restrict__ stf2, int4* __restrict__ posq2, double3 origin, double invq,
-                              const int* __restrict__ gate, int packed) {
+                              const int* __restrict__ gate, int packed, double4* __restrict__ xr2,
+                              double4* __restrict__ vp2) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n || (gate && *gate == 0)) return;
     int o = sorted[t];
@@ -568,6 +597,10 @@ __global__ void k_sph_permute(int n, const int* __restrict__ sorted, const doubl
     st2[t] = q;
     velf2[t] = packed ? velf_p(v, q) : f4(v);
     stf2[t] = f4(q);
+    if (xr2) {
+        xr2[t] = d4(xyz(p), q.x);
+        vp2[t] = d4(xyz(v), q.y);
+    }
     rho02[t] = rho0[o];
     drho2[t] = drho[o];
     id2[t] = id[o];
@@ -1306,49 +1339,99 @@ __global__ void __launch_bounds__(kSphBlock, kDensityBlocks<R>) k_sph_density(Sp
 // ---------------------------------------------------------------------------
 // Mixed-precision passes for scenes with uniform particle constants (UniK);
 // with markers (kMarkers) the shadows stay unpacked and the markers' terms
-// come from the general boundary functions.  Same pair sets, same formulas as k_sph_accel /
-// k_sph_density (updateWCSPHAccelerationKernel and
+// come from the general boundary functions.  Same pair sets, same formulas as
+// k_sph_accel / k_sph_density (updateWCSPHAccelerationKernel and
 // updateWCSPHDensityChangeKernel, WCSPHIntegrationKernel.cu:42-282), with
-// the constants hoisted and the terms regrouped:
-//   grad W_ij = K dq r'/|r'|,  dq = 2 t^3 (t - 1 - 2 q_n),  t = max(1 - q_n/2, 0);
-//   U_L - U_R = -(v_i - v_j) . r'/|r'|;
-//   r_hat . grad W = K dq (the reference's viscosity factor, Q5);
-//   momentum:   a_i += s [2 nu m (v_i - v_j) - 2 m P* r'/|r'|],  s = K dq / (rho_i rho_j);
-//   continuity: (v_i - v*) . grad W = K dq [(v_i - v_j) . r'/|r'| + (P_L - P_R) / (rho_bar c_bar)] / 2.
+// the constants hoisted and the terms regrouped.  With t = max(1 - q_n / 2, 0)
+// the Wendland factor 2 t^3 (t - 1 - 2 q_n) is -5 t^3 q_n, so
+//   grad W_ij = f r',  f = fC t^3  (r' in position quanta, no division by |r'|);
+//   r_hat . grad W = f |r'| (the reference's viscosity factor, Q5);
+//   U_L - U_R = (v_j - v_i) . r' / |r'|;
+//   momentum:   a_i += f / (rho_i rho_j) [-2 m P* r' - 2 nu m |r'| (v_j - v_i)];
+//   continuity: (v_i - v*) . grad W / rho_j = f [|r'| (P_L - P_R) 2 / c
+//               - (rho_i + rho_j) (v_j - v_i) . r'] / (2 rho_j (rho_i + rho_j)).
+// A lane takes its neighbours two at a time in packed FP32 (add / mul / fma
+// .f32x2: one issue for both).  A dam
+// break of 128,000 against one neighbour at a time: first pass 64.7 -> 63.5 us,
+// second 46.2 -> 38.6, continuity 45.4 -> 40.5; of a million 424 -> 431,
+// 327 -> 270, 315 -> 277.  What is left waits for the gathers (7 of 13 stalled
+// warps, L1 at 62% of its data wavefronts, 42% of the issue slots).
 // The fluid shadows are packed (k_sph_pack): the fixed-point position
 // carries rho in w and the FP32 velocity carries p, so a fluid neighbour is
 // two 16-byte gathers (the general passes gather a third record, the FP32
 // state); a dummy is three (position, velocity, normal).  Each pass writes
 // the packed shadows of the records it writes; the continuity pass, which
-// changes rho and p, writes the next position / velocity buffers.
+// changes rho and p, writes the next buffers of the shadows alone.
+__device__ __forceinline__ float2 two(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// -1 / x: the approximation y with one Newton step, y (x y - 2).  (Densities
+// are nearly uniform, so an approximation's error has one sign over all pairs
+// and steps, as a constant's rounding has; UniK.)
+__device__ __forceinline__ float2 nrcp2(float2 x) {
+    const float2 y = make_float2(rcp_approx(x.x), rcp_approx(x.y));
+    return __fmul2_rn(y, __ffma2_rn(x, y, two(-2.0f)));
+}
+// kLanes lanes share a particle: a quad, or in a small scene, whose quads do
+// not fill the GPU and which waits for a quad's chain of some twenty
+// neighbours, four quads that take every fourth pair of row entries.
+// 1,000 particles: first pass, second and continuity 18.0, 10.9
+// and 10.8 us on quads, one neighbour at a time, 7.1, 4.4 and 4.5 so; 18,000 in
+// FP64 were slower (79.9 us a step against 74.7).
+constexpr int kWide = 16;
+constexpr int kWideFluid = 8192;  // largest fluid that runs on kWide lanes per particle
+template <int kLanes>
+__device__ __forceinline__ int uni_particle() {
+    return (int)(blockIdx.x * (kSphBlock / kLanes) + threadIdx.x / kLanes);
+}
+template <int kLanes>
+__device__ __forceinline__ unsigned lanes_mask() {
+    return ((1u << kLanes) - 1u) << ((threadIdx.x & 31) & ~(unsigned)(kLanes - 1));
+}
+template <int kLanes, class T>
+__device__ __forceinline__ T lanes_sum(T v, unsigned m) {
+#pragma unroll
+    for (int o = 1; o < kLanes; o <<= 1) v += __shfl_xor_sync(m, v, o);
+    return v;
+}
 
+// Two neighbours: r' and its derived factors.
 struct PairGeom {
-    float3 r;   // r_i - r_j in quanta
-    float inv_r;
-    float Kdq;  // K dq(q_n)
+    float2 x, y, z;  // r_i - r_j in quanta
+    float2 r2, inv, r;  // |r'|^2, 1 / |r'|, |r'|
+    float2 f;        // grad W / r'
 };
-__device__ __forceinline__ PairGeom pair_geom(const int4& qi, const int4& qj, const UniK& u) {
+__device__ __forceinline__ float quanta(int a, int b) { return (float)(int)((unsigned)a - (unsigned)b); }
+__device__ __forceinline__ PairGeom pair_geom(const int4& q, const int4& a, const int4& b, const UniK& u) {
     PairGeom p;
-    p.r = make_float3((float)(int)((unsigned)qi.x - (unsigned)qj.x), (float)(int)((unsigned)qi.y - (unsigned)qj.y),
-                      (float)(int)((unsigned)qi.z - (unsigned)qj.z));
-    const float r2 = dot(p.r, p.r);
-    p.inv_r = rsqrtf(fmaxf(r2, 1e-30f));
-    const float qn = r2 * p.inv_r * u.invhq;
-    const float t = fmaxf(1.0f - 0.5f * qn, 0.0f);
-    const float t3 = t * t * t;
-    p.Kdq = u.K * (2.0f * t3 * (t - 1.0f - 2.0f * qn));
+    p.x = make_float2(quanta(q.x, a.x), quanta(q.x, b.x));
+    p.y = make_float2(quanta(q.y, a.y), quanta(q.y, b.y));
+    p.z = make_float2(quanta(q.z, a.z), quanta(q.z, b.z));
+    p.r2 = __ffma2_rn(p.x, p.x, __ffma2_rn(p.y, p.y, __fmul2_rn(p.z, p.z)));
+    p.inv = make_float2(rsqrt_approx(fmaxf(p.r2.x, 1e-30f)), rsqrt_approx(fmaxf(p.r2.y, 1e-30f)));
+    p.r = __fmul2_rn(p.r2, p.inv);
+    float2 t = __ffma2_rn(p.r, u.mh, two(1.0f));
+    t = make_float2(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f));
+    p.f = __fmul2_rn(__fmul2_rn(__fmul2_rn(t, t), t), u.fC);
     return p;
 }
 // The reference's cutoff test for a skin candidate, from the quanta
 // difference: FP32 outside a band of 2e-6 cut^2, the FP64 test on the FP64
 // positions inside it (as cutoff_f).
-__device__ __forceinline__ bool cutoff_u(const float3& r, const UniK& u, const double4& pi,
-                                         const double4* __restrict__ other, int j) {
-    const float d2 = dot(r, r);
+__device__ __forceinline__ bool cutoff_u(float d2, const UniK& u, const double4* __restrict__ own,
+                                         const double4* __restrict__ other, int i, int j) {
     const float band = 2.0e-6f * u.c2q;
     if (d2 < u.c2q - band) return true;
     if (d2 > u.c2q + band) return false;
-    const double4 pj = other[j];
+    const double4 pi = own[i], pj = other[j];
     const double cd = 2.0 * fmax(pi.w, pj.w);
     const double3 dr = xyz(pi) - xyz(pj);
     return (cd * cd - dot(dr, dr)) >= 0.;
@@ -1382,98 +1465,247 @@ __device__ __forceinline__ float4 nb_vp(const SphDev& d, int j, const int4& qj, 
         return v;
     }
 }
-// vj = (v_j, p_j), rhoj from the packed shadows
-__device__ __forceinline__ void acc_fluid_u(const OwnU& o, const PairGeom& p, const float4& vj, float rhoj,
-                                            const UniK& u, float3& acc) {
-    const float3 dv = o.v - make_float3(vj.x, vj.y, vj.z);
-    const float dU = -dot(dv, p.r) * p.inv_r;
-    const float beta = fminf(3.0f * fmaxf(dU, 0.0f), u.cF);
-    const float Ps = 0.5f * (o.PL + vj.w) + 0.5f * beta * (0.5f * (o.rho + rhoj)) * dU;
-    const float s = p.Kdq * __fdividef(1.0f, o.rho * rhoj);
-    const float sw = s * u.mF2 * Ps * p.inv_r;
-    const float sb = s * u.bF;
-    acc += sb * dv - sw * p.r;
+struct Acc2 {
+    float2 x, y, z;
+};
+__device__ __forceinline__ double3 acc2_sum(const Acc2& a) {
+    return mk3((double)a.x.x + (double)a.x.y, (double)a.y.x + (double)a.y.y, (double)a.z.x + (double)a.z.y);
 }
-// The dummy's extrapolated pressure and density (WCSPHIntegrationKernel.cu:
+// The sum times r, as an accumulator again: between the fluid's and the dummies'
+// terms (in FP64 the fluid's sum would hold six registers through the dummy
+// loop: second pass at 128,000 40.1 us against 38.6).
+__device__ __forceinline__ Acc2 acc2_scaled(const Acc2& a, double r) {
+    const double3 t = r * acc2_sum(a);
+    return Acc2{make_float2((float)t.x, 0.f), make_float2((float)t.y, 0.f), make_float2((float)t.z, 0.f)};
+}
+// v_j - v_i of two neighbours.
+__device__ __forceinline__ void rel_vel(const OwnU& o, const float4& a, const float4& b, float2& x, float2& y, float2& z) {
+    x = make_float2(a.x - o.v.x, b.x - o.v.x);
+    y = make_float2(a.y - o.v.y, b.y - o.v.y);
+    z = make_float2(a.z - o.v.z, b.z - o.v.z);
+}
+// Momentum of two pairs with the Riemann velocity jump dU = U_L - U_R and the
+// neighbours' P and rho: beta = min(3 max(dU, 0), c), P* = (P_L + P_R) / 2 +
+// beta (rho_i + rho_j) / 2 dU / 2.
+__device__ __forceinline__ void add_momentum(const OwnU& o, const PairGeom& p, float2 dU, float2 P, float2 rho,
+                                             float2 dx, float2 dy, float2 dz, const float2& c3, const float2& pm,
+                                             const float2& bm, float c, Acc2& acc) {
+    const float2 up = make_float2(fmaxf(dU.x, 0.0f), fmaxf(dU.y, 0.0f));
+    float2 beta = __fmul2_rn(up, c3);
+    beta = make_float2(fminf(beta.x, c), fminf(beta.y, c));
+    const float2 jump = __fmul2_rn(__fmul2_rn(beta, up), __fadd2_rn(rho, two(o.rho)));
+    // 2 m P* = pm (P_L + P_R + beta (rho_i + rho_j) dU / 2)
+    const float2 Ps = __fmul2_rn(pm, __ffma2_rn(jump, two(0.5f), __fadd2_rn(P, two(o.PL))));
+    const float2 rr = __fmul2_rn(rho, two(o.rho));
+    const float2 s = __fmul2_rn(p.f, nrcp2(rr));
+    const float2 sw = __fmul2_rn(s, Ps), sb = __fmul2_rn(__fmul2_rn(s, p.r), bm);
+    acc.x = __ffma2_rn(sb, dx, __ffma2_rn(sw, p.x, acc.x));
+    acc.y = __ffma2_rn(sb, dy, __ffma2_rn(sw, p.y, acc.y));
+    acc.z = __ffma2_rn(sb, dz, __ffma2_rn(sw, p.z, acc.z));
+}
+// va, vb = (v_j, p_j)
+__device__ __forceinline__ void acc_fluid_u(const OwnU& o, const PairGeom& p, const float4& va, const float4& vb,
+                                            float rhoa, float rhob, const UniK& u, Acc2& acc) {
+    float2 dx, dy, dz;
+    rel_vel(o, va, vb, dx, dy, dz);
+    const float2 dU = __fmul2_rn(__ffma2_rn(dx, p.x, __ffma2_rn(dy, p.y, __fmul2_rn(dz, p.z))), p.inv);
+    add_momentum(o, p, dU, make_float2(va.w, vb.w), make_float2(rhoa, rhob), dx, dy, dz, u.c3, u.pF, u.bF, u.cF, acc);
+}
+// The dummies' extrapolated pressure and density (WCSPHIntegrationKernel.cu:
 // 110-143): P_R = P_L + rho_i max(-g . r_ij, 0), rho_j = P_R / c_j^2 + rho0_j.
-__device__ __forceinline__ void dummy_state_u(const OwnU& o, const PairGeom& p, const UniK& u, float& PR, float& rhoj) {
-    const float grj = fmaxf(-dot(u.gq, p.r), 0.0f);
-    PR = o.PL + o.rho * grj;
-    rhoj = PR * u.invcD2 + u.rho0D;
+__device__ __forceinline__ void dummy_state_u(const OwnU& o, const PairGeom& p, const UniK& u, float2& PR, float2& rho) {
+    const float2 gr = __ffma2_rn(p.x, two(u.gq.x), __ffma2_rn(p.y, two(u.gq.y), __fmul2_rn(p.z, two(u.gq.z))));
+    const float2 up = make_float2(fmaxf(-gr.x, 0.0f), fmaxf(-gr.y, 0.0f));
+    PR = __ffma2_rn(up, two(o.rho), two(o.PL));
+    rho = __ffma2_rn(PR, two(u.invcD2), two(u.rho0D));
 }
-__device__ __forceinline__ void acc_dummy_u(const OwnU& o, const PairGeom& p, const float4& vj, const float4& nj,
-                                            const UniK& u, float3& acc) {
-    const float3 vd = make_float3(vj.x, vj.y, vj.z), nw = make_float3(nj.x, nj.y, nj.z);
-    const float UL = -dot(nw, o.v);
-    const float UR = -UL - 2.0f * dot(nw, vd);
-    float PR, rhoj;
-    dummy_state_u(o, p, u, PR, rhoj);
-    const float dU = UL - UR;
-    const float beta = fminf(3.0f * fmaxf(dU, 0.0f), u.cbarD);
-    const float Ps = 0.5f * (o.PL + PR) + 0.5f * beta * (0.5f * (o.rho + rhoj)) * dU;
-    const float s = p.Kdq * __fdividef(1.0f, o.rho * rhoj);
-    const float sw = s * u.mD2 * Ps * p.inv_r;
-    const float sb = s * u.bD;
-    acc += sb * (o.v - vd) - sw * p.r;
+// U_L - U_R = 2 n . (v_dummy - v_i)
+__device__ __forceinline__ void acc_dummy_u(const OwnU& o, const PairGeom& p, const float4& va, const float4& vb,
+                                            const float4& na, const float4& nb, const UniK& u, Acc2& acc) {
+    float2 dx, dy, dz, PR, rho;
+    rel_vel(o, va, vb, dx, dy, dz);
+    const float2 dn = __ffma2_rn(dx, make_float2(na.x, nb.x),
+                                 __ffma2_rn(dy, make_float2(na.y, nb.y), __fmul2_rn(dz, make_float2(na.z, nb.z))));
+    dummy_state_u(o, p, u, PR, rho);
+    add_momentum(o, p, __fadd2_rn(dn, dn), PR, rho, dx, dy, dz, u.c3, u.pD, u.bD, u.cbarD, acc);
+}
+// f |r'| (P_R - P_L) 2 / c + f (rho_i + rho_j) (v_j - v_i) . r', over
+// -rho_j (rho_i + rho_j): twice the continuity term without the mass.
+__device__ __forceinline__ void add_continuity(const OwnU& o, const PairGeom& p, const float4& va, const float4& vb,
+                                               float2 P, float2 rho, const float2& dc, float2& sum) {
+    float2 dx, dy, dz;
+    rel_vel(o, va, vb, dx, dy, dz);
+    const float2 w = __ffma2_rn(dx, p.x, __ffma2_rn(dy, p.y, __fmul2_rn(dz, p.z)));
+    const float2 rs = __fadd2_rn(rho, two(o.rho));
+    const float2 num = __ffma2_rn(__fmul2_rn(__fadd2_rn(P, two(-o.PL)), dc), p.r, __fmul2_rn(rs, w));
+    sum = __ffma2_rn(__fmul2_rn(p.f, num), nrcp2(__fmul2_rn(rho, rs)), sum);
 }
 
-// Resident blocks: the first pass (skin rows) fits 48 registers without
-// spilling and gains from the extra warps (10 blocks: 70 -> 66 us at 128k);
-// the second pass keeps 64 (at 48 it spills).  kMarkers: a coupled scene
-// (unpacked shadows; the markers' terms by the general boundary functions,
-// the same pairs and terms as the general passes and the reaction kernel),
-// at 8 blocks despite a few spills (ice sheet 5.4-5.6 ms per coupled step at
-// 7 blocks, 5.1-5.2 at 8; 6 and 9 blocks no better).
-template <bool kSkin, bool kMarkers>
-constexpr int kUniAccelBlocks = kMarkers ? 8 : (kSkin ? 10 : 8);
-template <bool kSkin, bool kMarkers = false>
-__global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
-    k_sph_accel_u(SphDev d, double hdt, double dt, int first) {
-    const int i = blockIdx.x * kSphPerBlock + threadIdx.x / kQuad;
-    if (i >= d.N) return;
-    const int sub = threadIdx.x & 3;
-    const unsigned gm = quad_mask();
-    const UniK& u = d.uk;
-    const double4 pi4 = d.pos[i];
-    const OwnU o = own_u(d, i);
-    float3 acc = make_float3(0.f, 0.f, 0.f);
-    if constexpr (kSkin) {
-        skin_loop(d.cntV[i], d.nbV, d.KF, i, d.nbF, d.cntF, pi4, d.g, d.fStart, d.pos, i, [&](int j) {
-            const int4 qj = d.posq[j];
-            const PairGeom p = pair_geom(o.q, qj, u);
-            if (!cutoff_u(p.r, u, pi4, d.pos, j)) return false;
-            float rhoj;
-            const float4 vj = nb_vp<kMarkers>(d, j, qj, rhoj);
-            acc_fluid_u(o, p, vj, rhoj, u, acc);
-            return true;
+// This lane's neighbours two at a time: f(a, b, two) with b = a and two =
+// false for an odd last one (quad_neighbors' rows and its overflow walk).
+template <int kLanes, class F>
+__device__ __forceinline__ void lane_pairs(int cnt, const int* __restrict__ nb, int K, int i, int self,
+                                           const double4* __restrict__ own, const GridDesc& g,
+                                           const int* __restrict__ cellStart, const double4* __restrict__ other, F&& f) {
+    const int sub = threadIdx.x & 3, seg = threadIdx.x % kLanes / kQuad;
+    constexpr int kStep = 2 * (kLanes / kQuad);
+    if (cnt >= 0) {
+        const int* __restrict__ row = nb + row_base(i, K) + sub;
+        const int mend = lane_count(cnt, sub);
+        int m = 2 * seg;
+        int j0 = m < mend ? __ldg(row + 32 * m) : -1;
+        int j1 = m + 1 < mend ? __ldg(row + 32 * (m + 1)) : -1;
+        for (; m < mend; m += kStep) {
+            const int a = j0, b = j1;
+            const int mn = m + kStep;
+            j0 = mn < mend ? __ldg(row + 32 * mn) : -1;
+            j1 = mn + 1 < mend ? __ldg(row + 32 * (mn + 1)) : -1;
+            f(a, b >= 0 ? b : a, b >= 0);
+        }
+        return;
+    }
+    const double4 pi = own[i];
+    const double3 ri = xyz(pi);
+    const Stencil st = stencil_of(ri, g);
+    for_stencil_rows(st, g, cellStart, [&](int b, int e) {
+        for (int j = b + threadIdx.x % kLanes; j < e; j += kLanes) {
+            if (j == self) continue;
+            const double4 pj = other[j];
+            const double cut = 2.0 * fmax(pi.w, pj.w);
+            const double3 r = ri - xyz(pj);
+            if ((cut * cut - dot(r, r)) >= 0.) f(j, j, false);
+        }
+    });
+}
+// skin_loop (first pass of a step) two candidates at a time: f(a, b, two, ka,
+// kb) tests the exact cutoff and adds the terms of the pairs that pass.  With
+// several quads on a row a prefix over them places each kept pair.
+template <int kLanes, class F>
+__device__ __forceinline__ void skin_pairs(int cnt, const int* __restrict__ nbV, int K, int i, int* __restrict__ nbOut,
+                                           int* __restrict__ cntOut, const double4* __restrict__ own, const GridDesc& g,
+                                           const int* __restrict__ cellStart, int self, F&& f) {
+    const int lig = threadIdx.x % kLanes, sub = threadIdx.x & 3, seg = lig / kQuad;
+    constexpr int kStep = 2 * (kLanes / kQuad);
+    bool ka, kb;
+    if (cnt < 0) {
+        if (lig == 0) cntOut[i] = -1;
+        const Stencil st = stencil_of(xyz(own[i]), g);
+        for_stencil_rows(st, g, cellStart, [&](int b, int e) {
+            for (int j = b + lig; j < e; j += kLanes)
+                if (j != self) f(j, j, false, ka, kb);
         });
-        if (d.ND > 0) {
-            skin_loop(d.cntVD[i], d.nbVD, d.KD, i, d.nbD, d.cntD, pi4, d.g, d.dStart, d.dpos, -1, [&](int j) {
-                const PairGeom p = pair_geom(o.q, d.dposq[j], u);
-                if (!cutoff_u(p.r, u, pi4, d.dpos, j)) return false;
-                acc_dummy_u(o, p, d.dvelf[j], d.dnormf[j], u, acc);
-                return true;
-            });
+        return;
+    }
+    const int* __restrict__ row = nbV + row_base(i, K) + sub;
+    int* __restrict__ out = nbOut + row_base(i, K) + sub;
+    int w = 0;  // pairs kept in this lane row so far
+    const int mend = lane_count(cnt, sub);
+    const unsigned gm = lanes_mask<kLanes>();
+    if constexpr (kLanes == kQuad) {
+        int m = 0;
+        int j0 = m < mend ? __ldg(row) : -1;
+        int j1 = m + 1 < mend ? __ldg(row + 32) : -1;
+        for (; m < mend; m += 2) {
+            const int a = j0, b = j1;
+            const int mn = m + 2;
+            j0 = mn < mend ? __ldg(row + 32 * mn) : -1;
+            j1 = mn + 1 < mend ? __ldg(row + 32 * (mn + 1)) : -1;
+            f(a, b >= 0 ? b : a, b >= 0, ka, kb);
+            if (ka) out[32 * w++] = a;
+            if (kb) out[32 * w++] = b;
         }
     } else {
-        quad_neighbors(d.cntF[i], d.nbF, d.KF, i, i, pi4, d.g, d.fStart, d.pos, [&](int j) {
-            const int4 qj = d.posq[j];
-            const PairGeom p = pair_geom(o.q, qj, u);
-            float rhoj;
-            const float4 vj = nb_vp<kMarkers>(d, j, qj, rhoj);
-            acc_fluid_u(o, p, vj, rhoj, u, acc);
-        });
+        const int all = (cnt + 3) >> 2;  // the longest of the four lane rows
+        for (int m0 = 0; m0 < all; m0 += kStep) {
+            const int m = m0 + 2 * seg;
+            const int a = m < mend ? __ldg(row + 32 * m) : -1;
+            const int b = m + 1 < mend ? __ldg(row + 32 * (m + 1)) : -1;
+            ka = kb = false;
+            if (a >= 0) f(a, b >= 0 ? b : a, b >= 0, ka, kb);
+            const int c = (ka ? 1 : 0) + (kb ? 1 : 0);
+            int incl = c;
+#pragma unroll
+            for (int o = kQuad; o < kLanes; o <<= 1) {
+                const int v = __shfl_up_sync(gm, incl, o, kLanes);
+                if (lig >= o) incl += v;
+            }
+            const int sum = __shfl_sync(gm, incl, kLanes - kQuad + sub, kLanes);
+            int at = w + incl - c;
+            if (ka) out[32 * at++] = a;
+            if (kb) out[32 * at] = b;
+            w += sum;
+        }
+    }
+    const unsigned qm = quad_mask();
+    const int over = quad_sum(w > 127 ? 1 : 0, qm);
+    const int lanes = quad_sum(w << (7 * sub), qm);
+    if (lig == 0) cntOut[i] = over ? -1 : (kLaneRows | lanes);
+}
+
+// Resident blocks.  The first pass spills in its loops beyond 8 (128,000:
+// 58 us at 8, 61 at 9, 73 at 10); the second fits 9 (a million: 296 us at 8, 280
+// at 9, 296 at 10).
+template <bool kSkin, bool kMarkers>
+constexpr int kUniAccelBlocks = kMarkers || kSkin ? 8 : 9;
+template <bool kSkin, bool kMarkers = false, int kLanes = kQuad>
+__global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
+    k_sph_accel_u(SphDev d, double hdt, double dt, int first) {
+    const int i = uni_particle<kLanes>();
+    if (i >= d.N) return;
+    const int sub = threadIdx.x % kLanes;
+    const unsigned gm = lanes_mask<kLanes>();
+    const UniK& u = d.uk;
+    const OwnU o = own_u(d, i);
+    const float2 z2 = make_float2(0.f, 0.f);
+    Acc2 acc2{z2, z2, z2};
+    if constexpr (kSkin) {
+        skin_pairs<kLanes>(d.cntV[i], d.nbV, d.KF, i, d.nbF, d.cntF, d.pos, d.g, d.fStart, i,
+                   [&](int a, int b, bool two, bool& ka, bool& kb) {
+                       const int4 qa = d.posq[a], qb = d.posq[b];
+                       float rhoa, rhob;
+                       const float4 va = nb_vp<kMarkers>(d, a, qa, rhoa), vb = nb_vp<kMarkers>(d, b, qb, rhob);
+                       PairGeom p = pair_geom(o.q, qa, qb, u);
+                       ka = cutoff_u(p.r2.x, u, d.pos, d.pos, i, a);
+                       kb = two && cutoff_u(p.r2.y, u, d.pos, d.pos, i, b);
+                       p.f = make_float2(ka ? p.f.x : 0.f, kb ? p.f.y : 0.f);
+                       acc_fluid_u(o, p, va, vb, rhoa, rhob, u, acc2);
+                   });
+        acc2 = acc2_scaled(acc2, u.aR);
         if (d.ND > 0) {
-            quad_neighbors(d.cntD[i], d.nbD, d.KD, i, -1, pi4, d.g, d.dStart, d.dpos, [&](int j) {
-                const PairGeom p = pair_geom(o.q, d.dposq[j], u);
-                acc_dummy_u(o, p, d.dvelf[j], d.dnormf[j], u, acc);
+            skin_pairs<kLanes>(d.cntVD[i], d.nbVD, d.KD, i, d.nbD, d.cntD, d.pos, d.g, d.dStart, -1,
+                       [&](int a, int b, bool two, bool& ka, bool& kb) {
+                           PairGeom p = pair_geom(o.q, d.dposq[a], d.dposq[b], u);
+                           ka = cutoff_u(p.r2.x, u, d.pos, d.dpos, i, a);
+                           kb = two && cutoff_u(p.r2.y, u, d.pos, d.dpos, i, b);
+                           p.f = make_float2(ka ? p.f.x : 0.f, kb ? p.f.y : 0.f);
+                           acc_dummy_u(o, p, d.dvelf[a], d.dvelf[b], d.dnormf[a], d.dnormf[b], u, acc2);
+                       });
+        }
+    } else {
+        lane_pairs<kLanes>(d.cntF[i], d.nbF, d.KF, i, i, d.pos, d.g, d.fStart, d.pos, [&](int a, int b, bool two) {
+            const int4 qa = d.posq[a], qb = d.posq[b];
+            float rhoa, rhob;
+            const float4 va = nb_vp<kMarkers>(d, a, qa, rhoa), vb = nb_vp<kMarkers>(d, b, qb, rhob);
+            PairGeom p = pair_geom(o.q, qa, qb, u);
+            p.f.y = two ? p.f.y : 0.f;
+            acc_fluid_u(o, p, va, vb, rhoa, rhob, u, acc2);
+        });
+        acc2 = acc2_scaled(acc2, u.aR);
+        if (d.ND > 0) {
+            lane_pairs<kLanes>(d.cntD[i], d.nbD, d.KD, i, -1, d.pos, d.g, d.dStart, d.dpos, [&](int a, int b, bool two) {
+                PairGeom p = pair_geom(o.q, d.dposq[a], d.dposq[b], u);
+                p.f.y = two ? p.f.y : 0.f;
+                acc_dummy_u(o, p, d.dvelf[a], d.dvelf[b], d.dnormf[a], d.dnormf[b], u, acc2);
             });
         }
     }
+    double3 a = u.aD * acc2_sum(acc2);
+    float3 acc = make_float3(0.f, 0.f, 0.f);
     if constexpr (kMarkers) {
         // as k_sph_accel: the fluid-marker skin row with the exact test the
         // reaction on the markers applies, or this step's rows (an overflowed
         // row walks the marker cells at the rows' build positions)
+        const double4 pi4 = d.pos[i];
         const FluidOwn<float> fo = fluid_own<float>(d, i, pi4, d.vel[i], d.st[i]);
         const BView mv = marker_view(d);
         const float3 g = cvt<float>(d.gravity);
@@ -1492,15 +1724,16 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
                            [&](int j) { boundary_acc<float>(d, fo, mv, j, g, acc); });
         }
     }
-    double3 a = up(acc);
-    a.x = quad_sum(a.x, gm);
-    a.y = quad_sum(a.y, gm);
-    a.z = quad_sum(a.z, gm);
+    if constexpr (kMarkers) a += up(acc);
+    a.x = lanes_sum<kLanes>(a.x, gm);
+    a.y = lanes_sum<kLanes>(a.y, gm);
+    a.z = lanes_sum<kLanes>(a.z, gm);
     if (sub != 0) return;
+    const double4 pi4 = d.pos[i];
     const double4 vi4 = d.vel[i];
     const double4 s4 = d.st[i];
     a += d.gravity;
-    d.acc[i] = d4(a, 0);
+    if (!first) d.acc[i] = d4(a, 0);  // (the second pass overwrites the first one's)
     const double3 v = xyz(vi4) + hdt * a;
     const double4 v4 = d4(v, vi4.w);
     d.velOut[i] = v4;
@@ -1516,51 +1749,46 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
     }
 }
 
-template <bool kMarkers = false>
+template <bool kMarkers = false, int kLanes = kQuad>
 __global__ void __launch_bounds__(kSphBlock, 8) k_sph_density_u(SphDev d, double dt) {
-    const int i = blockIdx.x * kSphPerBlock + threadIdx.x / kQuad;
+    const int i = uni_particle<kLanes>();
     if (i >= d.N) return;
-    const int sub = threadIdx.x & 3;
-    const unsigned gm = quad_mask();
+    const int sub = threadIdx.x % kLanes;
+    const unsigned gm = lanes_mask<kLanes>();
     const UniK& u = d.uk;
-    const double4 pi4 = d.pos[i];
     const OwnU o = own_u(d, i);
-    float sumF = 0.f, sumD = 0.f;  // sum of (1 / rho_j) (v_i - v*) . grad W / (1/2), per kind of neighbour
-    quad_neighbors(d.cntF[i], d.nbF, d.KF, i, i, pi4, d.g, d.fStart, d.pos, [&](int j) {
-        const int4 qj = d.posq[j];
-        const PairGeom p = pair_geom(o.q, qj, u);
-        float rhoj;
-        const float4 vj = nb_vp<kMarkers>(d, j, qj, rhoj);  // (v_j, p_j)
-        const float3 dv = o.v - make_float3(vj.x, vj.y, vj.z);
-        const float rbar = 0.5f * (o.rho + rhoj);
-        const float X = __fdividef(o.PL - vj.w, rbar * u.cF);
-        sumF += __fdividef(p.Kdq * (dot(dv, p.r) * p.inv_r + X), rhoj);
+    // sums of twice the terms over their masses, per kind of neighbour
+    float2 sumF = make_float2(0.f, 0.f), sumD = make_float2(0.f, 0.f);
+    lane_pairs<kLanes>(d.cntF[i], d.nbF, d.KF, i, i, d.pos, d.g, d.fStart, d.pos, [&](int a, int b, bool two) {
+        const int4 qa = d.posq[a], qb = d.posq[b];
+        float rhoa, rhob;
+        const float4 va = nb_vp<kMarkers>(d, a, qa, rhoa), vb = nb_vp<kMarkers>(d, b, qb, rhob);  // (v_j, p_j)
+        PairGeom p = pair_geom(o.q, qa, qb, u);
+        p.f.y = two ? p.f.y : 0.f;
+        add_continuity(o, p, va, vb, make_float2(va.w, vb.w), make_float2(rhoa, rhob), u.dF, sumF);
     });
     if (d.ND > 0) {
-        quad_neighbors(d.cntD[i], d.nbD, d.KD, i, -1, pi4, d.g, d.dStart, d.dpos, [&](int j) {
-            const PairGeom p = pair_geom(o.q, d.dposq[j], u);
-            const float4 vj = d.dvelf[j];
-            float PR, rhoj;
-            dummy_state_u(o, p, u, PR, rhoj);
-            const float3 dv = o.v - make_float3(vj.x, vj.y, vj.z);
-            const float rbar = 0.5f * (o.rho + rhoj);
-            const float X = __fdividef(o.PL - PR, rbar * u.cbarD);
-            sumD += __fdividef(p.Kdq * (dot(dv, p.r) * p.inv_r + X), rhoj);
+        lane_pairs<kLanes>(d.cntD[i], d.nbD, d.KD, i, -1, d.pos, d.g, d.dStart, d.dpos, [&](int a, int b, bool two) {
+            PairGeom p = pair_geom(o.q, d.dposq[a], d.dposq[b], u);
+            p.f.y = two ? p.f.y : 0.f;
+            float2 PR, rho;
+            dummy_state_u(o, p, u, PR, rho);
+            add_continuity(o, p, d.dvelf[a], d.dvelf[b], PR, rho, u.dD, sumD);
         });
     }
     float dRhoM = 0.f;  // the markers' terms, as k_sph_density
     if constexpr (kMarkers) {
-        const FluidOwn<float> fo = fluid_own<float>(d, i, pi4, d.vel[i], d.st[i]);
+        const double4 pm = d.pos[i];
+        const FluidOwn<float> fo = fluid_own<float>(d, i, pm, d.vel[i], d.st[i]);
         const BView mv = marker_view(d);
         const float3 g = cvt<float>(d.gravity);
         const int cM = d.cntM[i];
-        quad_neighbors(cM, d.nbM, d.KM, i, -1, cM < 0 ? d.lpos[i] : pi4, d.g, d.mStart, d.mpos,
+        quad_neighbors(cM, d.nbM, d.KM, i, -1, cM < 0 ? d.lpos[i] : pm, d.g, d.mStart, d.mpos,
                        [&](int j) { boundary_drho<float>(d, fo, mv, j, g, dRhoM); });
     }
-    const double dsum =
-        quad_sum(0.5 * ((double)u.mF * (double)sumF + (double)u.mD * (double)sumD) + (double)dRhoM, gm);
+    const double dsum = lanes_sum<kLanes>(u.sF * ((double)sumF.x + (double)sumF.y) +
+                                 u.sD * ((double)sumD.x + (double)sumD.y) + (double)dRhoM, gm);
     if (sub != 0) return;
-    const double4 vi4 = d.vel[i];
     const double4 s4 = d.st[i];
     const double dr = dsum * (2.0 * (double)o.rho);
     double ch = d.drho[i] + dr * dt;
@@ -1571,12 +1799,216 @@ __global__ void __launch_bounds__(kSphBlock, 8) k_sph_density_u(SphDev d, double
     d.stOut[i] = so;
     d.stfOut[i] = f4(so);
     if constexpr (kMarkers) return;  // unpacked shadows: the state records alone change
-    // the next position / velocity buffers: the same records, their packed
-    // shadows with the new rho and p
-    d.posOut[i] = pi4;
-    d.velOut[i] = vi4;
+    // the packed shadows with the new rho and p
     d.posqOut[i] = make_int4(o.q.x, o.q.y, o.q.z, __float_as_int((float)so.x));
-    d.velfOut[i] = velf_p(vi4, so);
+    d.velfOut[i] = make_float4(o.v.x, o.v.y, o.v.z, (float)so.y);
+}
+
+// ---------------------------------------------------------------------------
+// FP64 passes for scenes with uniform particle constants and no markers: the
+// regrouped terms above in double precision, one neighbour at a time.  The
+// general FP64 passes are bound by the FP64 pipe and by their gathers (three
+// 32-byte records per fluid neighbour, four divisions or square roots per
+// pair); here a neighbour is two records (xr, vp), each one 32-byte load, and
+// a pair takes one reciprocal square root and one reciprocal.  128,000: first
+// pass 162 -> 95 us, second 127 -> 73, continuity 126 -> 68.  Side by side two
+// neighbours hold more registers: a fluid whose blocks all fit the GPU at four
+// per SM runs so (18,000: 20, 15 and 14 us; 74.7 -> 69.9 us a step), a larger
+// one at six (at four 311 us a step against 295).
+//
+// 1 / sqrt(x) and 1 / x from the FP32 approximation y0 (relative error below
+// 2^-21) by one step of Halley's respectively the cubic Newton-Schulz series in
+// e = 1 - x y0^2 (1 - x y0): what is left is of order e^3 < 2^-60.
+__device__ __forceinline__ double rsqrt_u(double x) {
+    const double y0 = (double)rsqrt_approx((float)x);
+    const double e = fma(-(x * y0), y0, 1.0);
+    return fma(y0 * e, fma(0.375, e, 0.5), y0);
+}
+__device__ __forceinline__ double rcp_u(double x) {
+    const double y0 = (double)rcp_approx((float)x);
+    const double e = fma(-x, y0, 1.0);
+    return fma(y0, fma(e, e, e), y0);
+}
+__device__ __forceinline__ double4 load32(const double4* __restrict__ p) {
+    double4 v;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
+}
+struct OwnD {
+    double3 x, v;
+    double rho, PL;
+};
+struct PairD {
+    double3 r;
+    double inv, len, f;
+};
+__device__ __forceinline__ OwnD own_d(const SphDev& d, int i) {
+    const double4 x = load32(d.xr + i), v = load32(d.vp + i);
+    return OwnD{xyz(x), xyz(v), x.w, v.w};
+}
+__device__ __forceinline__ PairD pair_geom_d(double3 r, double r2, const UniD& u) {
+    PairD p;
+    p.r = r;
+    p.inv = r2 < 1.0e-20 ? 0.0 : rsqrt_u(r2);
+    p.len = r2 * p.inv;
+    const double t = fmax(fma(p.len, u.mh, 1.0), 0.0);
+    p.f = u.fC * (t * t * t);
+    return p;
+}
+__device__ __forceinline__ void add_momentum_d(const OwnD& o, const PairD& p, double dU, double P, double rho, double3 dv,
+                                               double pm, double bm, double c, double3& acc) {
+    const double up = fmax(dU, 0.0);
+    const double beta = fmin(3.0 * up, c);
+    const double Ps = pm * fma(0.5 * beta * up, rho + o.rho, P + o.PL);
+    const double s = p.f * rcp_u(rho * o.rho);
+    const double sw = s * Ps, sb = s * p.len * bm;
+    acc.x = fma(sb, dv.x, fma(sw, p.r.x, acc.x));
+    acc.y = fma(sb, dv.y, fma(sw, p.r.y, acc.y));
+    acc.z = fma(sb, dv.z, fma(sw, p.r.z, acc.z));
+}
+__device__ __forceinline__ void dummy_state_d(const OwnD& o, const PairD& p, double3 g, const UniD& u, double& PR,
+                                              double& rho) {
+    PR = fma(fmax(-dot(g, p.r), 0.0), o.rho, o.PL);
+    rho = fma(PR, u.invcD2, u.rho0D);
+}
+__device__ __forceinline__ void acc_dummy_d(const SphDev& d, const OwnD& o, const PairD& p, int j, double3& acc) {
+    const double3 dv = xyz(load32(d.dvel + j)) - o.v;
+    const double3 n = xyz(load32(d.dnorm + j));
+    double PR, rho;
+    dummy_state_d(o, p, d.gravity, d.ud, PR, rho);
+    add_momentum_d(o, p, 2.0 * dot(n, dv), PR, rho, dv, d.ud.pD, d.ud.bD, d.ud.cbarD, acc);
+}
+__device__ __forceinline__ void add_continuity_d(const OwnD& o, const PairD& p, double3 dv, double P, double rho,
+                                                 double dc, double& sum) {
+    const double rs = rho + o.rho;
+    const double num = fma((P - o.PL) * dc, p.len, -(rs * dot(dv, p.r)));
+    sum = fma(p.f * num, rcp_u(rho * rs), sum);
+}
+
+template <bool kSkin, int kLanes = kQuad, int kBlocks = 6>
+__global__ void __launch_bounds__(kSphBlock, kBlocks) k_sph_accel_u64(SphDev d, double hdt, double dt, int first) {
+    const int i = uni_particle<kLanes>();
+    if (i >= d.N) return;
+    const int sub = threadIdx.x % kLanes;
+    const unsigned gm = lanes_mask<kLanes>();
+    const OwnD o = own_d(d, i);
+    double3 acc = mk3(0, 0, 0);
+    // two neighbours side by side, without a branch between them: their chains
+    // of FP64 operations overlap (a pair beyond the cutoff, or the missing second
+    // one, has its kernel factor zeroed)
+    auto fluid = [&](int a, int b, bool two, bool& ka, bool& kb) {
+        const double4 xa = load32(d.xr + a), xb = load32(d.xr + b);
+        const double4 va = load32(d.vp + a), vb = load32(d.vp + b);
+        const double3 ra = o.x - xyz(xa), rb = o.x - xyz(xb);
+        const double a2 = dot(ra, ra), b2 = dot(rb, rb);
+        ka = !kSkin || (d.ud.cut2 - a2) >= 0.;
+        kb = two && (!kSkin || (d.ud.cut2 - b2) >= 0.);
+        PairD p = pair_geom_d(ra, a2, d.ud), q = pair_geom_d(rb, b2, d.ud);
+        if (kSkin) p.f = ka ? p.f : 0.0;
+        q.f = kb ? q.f : 0.0;
+        const double3 da = xyz(va) - o.v, db = xyz(vb) - o.v;
+        add_momentum_d(o, p, dot(da, ra) * p.inv, va.w, xa.w, da, d.ud.pF, d.ud.bF, d.ud.cF, acc);
+        add_momentum_d(o, q, dot(db, rb) * q.inv, vb.w, xb.w, db, d.ud.pF, d.ud.bF, d.ud.cF, acc);
+    };
+    auto dummy = [&](int j) {
+        const double3 r = o.x - xyz(load32(d.dpos + j));
+        const double r2 = dot(r, r);
+        if (kSkin && !((d.ud.cut2 - r2) >= 0.)) return false;
+        acc_dummy_d(d, o, pair_geom_d(r, r2, d.ud), j, acc);
+        return true;
+    };
+    if constexpr (kSkin) {
+        skin_pairs<kLanes>(d.cntV[i], d.nbV, d.KF, i, d.nbF, d.cntF, d.pos, d.g, d.fStart, i, fluid);
+        if (d.ND > 0)
+            skin_pairs<kLanes>(d.cntVD[i], d.nbVD, d.KD, i, d.nbD, d.cntD, d.pos, d.g, d.dStart, -1,
+                       [&](int a, int b, bool two, bool& ka, bool& kb) {
+                           ka = dummy(a);
+                           kb = two && dummy(b);
+                       });
+    } else {
+        lane_pairs<kLanes>(d.cntF[i], d.nbF, d.KF, i, i, d.pos, d.g, d.fStart, d.pos, [&](int a, int b, bool two) {
+            bool ka, kb;
+            fluid(a, b, two, ka, kb);
+        });
+        if (d.ND > 0)
+            lane_pairs<kLanes>(d.cntD[i], d.nbD, d.KD, i, -1, d.pos, d.g, d.dStart, d.dpos, [&](int a, int b, bool two) {
+                dummy(a);
+                if (two) dummy(b);
+            });
+    }
+    acc.x = lanes_sum<kLanes>(acc.x, gm);
+    acc.y = lanes_sum<kLanes>(acc.y, gm);
+    acc.z = lanes_sum<kLanes>(acc.z, gm);
+    if (sub != 0) return;
+    const double4 vi4 = d.vel[i];
+    acc += d.gravity;
+    if (!first) d.acc[i] = d4(acc, 0);
+    const double3 v = xyz(vi4) + hdt * acc;
+    d.velOut[i] = d4(v, vi4.w);
+    d.vpOut[i] = d4(v, o.PL);
+    if (first) {
+        const double4 pi4 = d.pos[i];
+        const double3 x = xyz(pi4) + dt * v;
+        d.posOut[i] = d4(x, pi4.w);
+        d.xrOut[i] = d4(x, o.rho);
+        if constexpr (kSkin) {
+            const double3 dd = x - xyz(d.xb[i]);
+            atomicMax(d.maxd2 + (blockIdx.x & (kSkinSlots - 1)), __float_as_uint((float)dot(dd, dd)));
+        }
+    }
+}
+
+template <int kLanes = kQuad, int kBlocks = 6>
+__global__ void __launch_bounds__(kSphBlock, kBlocks) k_sph_density_u64(SphDev d, double dt) {
+    const int i = uni_particle<kLanes>();
+    if (i >= d.N) return;
+    const int sub = threadIdx.x % kLanes;
+    const unsigned gm = lanes_mask<kLanes>();
+    const OwnD o = own_d(d, i);
+    double sumF = 0, sumD = 0;
+    auto fluid = [&](int a, int b, bool two) {
+        const double4 xa = load32(d.xr + a), xb = load32(d.xr + b);
+        const double4 va = load32(d.vp + a), vb = load32(d.vp + b);
+        const double3 ra = o.x - xyz(xa), rb = o.x - xyz(xb);
+        const PairD p = pair_geom_d(ra, dot(ra, ra), d.ud);
+        PairD q = pair_geom_d(rb, dot(rb, rb), d.ud);
+        q.f = two ? q.f : 0.0;
+        add_continuity_d(o, p, xyz(va) - o.v, va.w, xa.w, d.ud.dF, sumF);
+        add_continuity_d(o, q, xyz(vb) - o.v, vb.w, xb.w, d.ud.dF, sumF);
+    };
+    auto dummy = [&](int j) {
+        const double3 r = o.x - xyz(load32(d.dpos + j));
+        const PairD p = pair_geom_d(r, dot(r, r), d.ud);
+        double PR, rho;
+        dummy_state_d(o, p, d.gravity, d.ud, PR, rho);
+        add_continuity_d(o, p, xyz(load32(d.dvel + j)) - o.v, PR, rho, d.ud.dD, sumD);
+    };
+    lane_pairs<kLanes>(d.cntF[i], d.nbF, d.KF, i, i, d.pos, d.g, d.fStart, d.pos, fluid);
+    if (d.ND > 0)
+        lane_pairs<kLanes>(d.cntD[i], d.nbD, d.KD, i, -1, d.pos, d.g, d.dStart, d.dpos, [&](int a, int b, bool two) {
+            dummy(a);
+            if (two) dummy(b);
+        });
+    const double dsum = lanes_sum<kLanes>(0.5 * (d.ud.mF * sumF + d.ud.mD * sumD), gm);
+    if (sub != 0) return;
+    const double4 s4 = d.st[i];
+    double ch = d.drho[i] + dsum * (2.0 * o.rho) * dt;
+    d.drho[i] = ch;
+    const double r0 = d.rho0[i];
+    if (ch < -0.1 * r0) ch = -0.1 * r0;
+    const double4 so = make_double4(ch + r0, s4.z * s4.z * ch, s4.z, s4.w);
+    d.stOut[i] = so;
+    d.xrOut[i] = d4(o.x, so.x);
+    d.vpOut[i] = d4(o.v, so.y);
+}
+// The gathered records of the FP64 passes from the particle records.
+__global__ void k_sph_pack64(int n, const double4* __restrict__ pos, const double4* __restrict__ vel,
+                             const double4* __restrict__ st, double4* __restrict__ xr, double4* __restrict__ vp) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const double4 q = st[t];
+    xr[t] = d4(xyz(pos[t]), q.x);
+    vp[t] = d4(xyz(vel[t]), q.y);
 }
 
 // Reaction of the fluid on the markers: for marker t, minus the sum over
@@ -1816,10 +2248,16 @@ struct SphScene {
     DBuf<float4> posf, dposf;
     DBuf<float4> velf[2], stf[2], dvelf, dstf, dnormf;  // FP32 shadows
     DBuf<int4> posq[2], dposq;                           // fixed-point positions
+    DBuf<double4> xr[2], vp[2];  // the specialised FP64 passes' records (buffers as pos, vel)
+    bool packed64 = false;       // ... are in use
     float q = 0;
     double invq = 0;
     float eps = 0;
     int P = 0, Vv = 0, S = 0, R0 = 0, D = 0, ID = 0;
+    // the gathered position and velocity records (posq, xr; velf, vp) have
+    // parities of their own: the specialised continuity pass renews them (they
+    // carry rho and p) without moving the particles
+    int QX = 0, QV = 0;
     int L = 0;  // pos buffer the current lists were built from
     DBuf<double4> dpos, dvel, dst, dnorm;
     DBuf<double> drhoD;  // dummy densities (normals only)
@@ -1885,19 +2323,61 @@ struct SphScene {
     // The uniform-constant passes (mixed precision); with markers they read
     // the unpacked shadows (packed only when nM == 0).
     bool uni_path() const { return uni.on && uniKernels && precision != DEMSPH_PRECISION_FP64; }
+    // The FP64 ones serve scenes without markers whose lengths and densities
+    // (and their squares) lie well inside the FP32 range: the passes start
+    // their reciprocals from FP32 approximations.
+    bool uni64_path() const {
+        if (!uni.on || !uniKernels || precision != DEMSPH_PRECISION_FP64 || nM > 0) return false;
+        const double sp = uni.h / 1.3, rho = uni.mF / (sp * sp * sp);
+        auto ok = [](double x) { return x > 1e-9 && x < 1e9; };
+        return ok(uni.h) && ok(rho) && (ND() == 0 || ok(uni.rho0D));
+    }
+    UniD uni_consts_d() const {
+        UniD k{};
+        const double h = uni.h, K = 21.0 / (16.0 * kPi * h * h * h * h), cd = 2.0 * h;
+        k.cut2 = cd * cd;
+        k.mh = -0.5 / h;
+        k.fC = -5.0 * K / h;
+        k.pF = -uni.mF;
+        k.bF = -2.0 * uni.nuF * uni.mF;
+        k.pD = -uni.mD;
+        k.bD = -2.0 * (0.5 * (uni.nuF + uni.nuD)) * uni.mD;
+        k.cF = uni.cF;
+        k.cbarD = 0.5 * (uni.cF + uni.cD);
+        k.dF = -2.0 / k.cF;
+        k.dD = -2.0 / k.cbarD;
+        k.mF = uni.mF;
+        k.mD = uni.mD;
+        k.invcD2 = uni.cD > 0 ? 1.0 / (uni.cD * uni.cD) : 0.0;
+        k.rho0D = uni.rho0D;
+        return k;
+    }
     UniK uni_consts() const {
         UniK k{};
         const double h = uni.h, qd = (double)q;
-        k.invhq = (float)(qd / h);
-        k.K = (float)(21.0 / (16.0 * kPi * h * h * h * h));
+        auto two = [](double x) { return make_float2((float)x, (float)x); };
+        const double K = 21.0 / (16.0 * kPi * h * h * h * h);
+        k.mh = two(-0.5 * qd / h);
+        k.fC = two(-5.0 * K * qd / h);
+        k.c3 = two(3.0);
+        k.pF = two(uni.mF);
+        k.bF = two(2.0 * uni.nuF * uni.mF);
+        k.pD = two(uni.mD);
+        k.bD = two(2.0 * (0.5 * (uni.nuF + uni.nuD)) * uni.mD);
+        k.dF = two(2.0 / uni.cF);
+        k.dD = two(2.0 / (0.5 * (uni.cF + uni.cD)));
+        // the rounding of mh (relative eps) scales t^3 at distance x 2 h by
+        // 1 - 3 eps x / (1 - x): weighted with the divergence sum's x^4 (1 - x)^3
+        // that is 1 - 5 eps
+        const double eps = (double)k.mh.x / (-0.5 * qd / h) - 1.0;
+        const double fix = (-5.0 * K * qd / h) / (double)k.fC.x * (1.0 + 5.0 * eps);
+        const double aF = fix * uni.mF / (double)k.pF.x;
+        k.aD = uni.mD > 0 ? fix * uni.mD / (double)k.pD.x : fix;
+        k.aR = aF / k.aD;
+        k.sF = 0.5 * fix * uni.mF;
+        k.sD = 0.5 * fix * uni.mD;
         k.c2q = (float)((2.0 * h / qd) * (2.0 * h / qd));
         k.cF = (float)uni.cF;
-        k.mF2 = (float)(2.0 * uni.mF);
-        k.bF = (float)(2.0 * uni.nuF * uni.mF);
-        k.mF = (float)uni.mF;
-        k.mD = (float)uni.mD;
-        k.mD2 = (float)(2.0 * uni.mD);
-        k.bD = (float)(2.0 * (0.5 * (uni.nuF + uni.nuD)) * uni.mD);
         k.cbarD = (float)(0.5 * (uni.cF + uni.cD));
         k.invcD2 = uni.cD > 0 ? (float)(1.0 / (uni.cD * uni.cD)) : 0.0f;
         k.rho0D = (float)uni.rho0D;
@@ -1942,8 +2422,8 @@ struct SphScene {
         d.pos = pos[P].p; d.lpos = pos[L].p; d.vel = vel[Vv].p; d.st = st[S].p; d.rho0 = rho0[R0].p; d.drho = drho[D].p;
         d.acc = acc.p;
         d.dpos = dpos.p; d.dvel = dvel.p; d.dst = dst.p; d.dnorm = dnorm.p;
-        d.velf = velf[Vv].p; d.stf = stf[S].p;
-        d.posq = posq[P].p; d.dposq = dposq.p; d.q = q; d.invq = invq;
+        d.velf = velf[QV].p; d.stf = stf[S].p;
+        d.posq = posq[QX].p; d.dposq = dposq.p; d.q = q; d.invq = invq;
         d.dvelf = dvelf.p; d.dstf = dstf.p; d.dnormf = dnormf.p;
         d.nbF = nbF.p; d.cntF = cntF.p; d.nbD = nbD.p; d.cntD = cntD.p;
         d.posf = posf.p; d.dposf = dposf.p; d.eps = eps;
@@ -1960,6 +2440,11 @@ struct SphScene {
         d.nbV = nbV.p; d.cntV = cntV.p; d.nbVD = nbVD.p; d.cntVD = cntVD.p;
         d.xb = xb.p; d.maxd2 = skinState.p ? skinState.p->maxd2 : nullptr;
         if (uni.on) d.uk = uni_consts();
+        if (packed64) {
+            d.ud = uni_consts_d();
+            d.xr = xr[QX].p;
+            d.vp = vp[QV].p;
+        }
         return d;
     }
 
@@ -2061,29 +2546,32 @@ struct SphScene {
         k_sph_permute<<<grid_for(n, 256), 256, 0, s>>>(n, fCells.sorted.p, pos[P].p, vel[Vv].p, st[S].p, rho0[R0].p,
                                                        drho[D].p, id[ID].p, pos[P ^ 1].p, vel[Vv ^ 1].p, st[S ^ 1].p,
                                                        rho0[R0 ^ 1].p, drho[D ^ 1].p, id[ID ^ 1].p, posf.p,
-                                                       velf[Vv ^ 1].p, stf[S ^ 1].p, posq[P ^ 1].p, fCells.g.mn,
-                                                       invq, gate, packed ? 1 : 0);
+                                                       velf[QV ^ 1].p, stf[S ^ 1].p, posq[QX ^ 1].p, fCells.g.mn,
+                                                       invq, gate, packed ? 1 : 0, packed64 ? xr[QX ^ 1].p : nullptr,
+                                                       packed64 ? vp[QV ^ 1].p : nullptr);
         if (gate) {  // a device-side decision: copy back instead of flipping the indices
             k_sph_copy_back<<<grid_for(n, 256), 256, 0, s>>>(
                 n, gate, pos[P ^ 1].p, vel[Vv ^ 1].p, st[S ^ 1].p, rho0[R0 ^ 1].p, drho[D ^ 1].p, id[ID ^ 1].p,
-                velf[Vv ^ 1].p, stf[S ^ 1].p, posq[P ^ 1].p, pos[P].p, vel[Vv].p, st[S].p, rho0[R0].p, drho[D].p,
-                id[ID].p, velf[Vv].p, stf[S].p, posq[P].p, xb.p);
+                velf[QV ^ 1].p, stf[S ^ 1].p, posq[QX ^ 1].p, pos[P].p, vel[Vv].p, st[S].p, rho0[R0].p, drho[D].p,
+                id[ID].p, velf[QV].p, stf[S].p, posq[QX].p, xb.p, packed64 ? xr[QX ^ 1].p : nullptr,
+                packed64 ? vp[QV ^ 1].p : nullptr, packed64 ? xr[QX].p : nullptr, packed64 ? vp[QV].p : nullptr);
             g_launches += 1;
         } else {
-            P ^= 1; Vv ^= 1; S ^= 1; R0 ^= 1; D ^= 1; ID ^= 1;
+            P ^= 1; Vv ^= 1; S ^= 1; R0 ^= 1; D ^= 1; ID ^= 1; QX ^= 1; QV ^= 1;
         }
         L = P;
     }
     // Rewrites the fluid shadows after a host-side change of the records.
     void refresh_shadows() {
         const int n = N();
-        k_sph_shadow<<<grid_for(n, 256), 256, 0, s>>>(n, vel[Vv].p, st[S].p, nullptr, velf[Vv].p, stf[S].p, nullptr);
-        k_sph_fix<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, fCells.g.mn, invq, posq[P].p);
+        k_sph_shadow<<<grid_for(n, 256), 256, 0, s>>>(n, vel[Vv].p, st[S].p, nullptr, velf[QV].p, stf[S].p, nullptr);
+        k_sph_fix<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, fCells.g.mn, invq, posq[QX].p);
         g_launches += 2;
         if (packed) {
-            k_sph_pack<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, vel[Vv].p, st[S].p, posq[P].p, velf[Vv].p, 1);
+            k_sph_pack<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, vel[Vv].p, st[S].p, posq[QX].p, velf[QV].p, 1);
             g_launches += 1;
         }
+        if (packed64) pack64();
         DEMSPH_LAUNCH_CHECK();
         skin_force();
     }
@@ -2091,14 +2579,33 @@ struct SphScene {
     // run (packed) or the general ones; called at the entry of every call
     // that launches the passes, outside any stream capture.
     bool packed = false;
+    void pack64() {
+        const int n = N();
+        k_sph_pack64<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, vel[Vv].p, st[S].p, xr[QX].p, vp[QV].p);
+        g_launches += 1;
+    }
     void sync_mode() {
+        const bool want64 = ready && uni64_path();
+        if (want64 != packed64) {
+            packed64 = want64;
+            graph.reset();
+            oneStepAfter.clear();
+            if (packed64) {
+                for (int b = 0; b < 2; b++) {
+                    if (xr[b].n < (size_t)N()) xr[b].alloc(N(), s, false);
+                    if (vp[b].n < (size_t)N()) vp[b].alloc(N(), s, false);
+                }
+                pack64();
+                DEMSPH_LAUNCH_CHECK();
+            }
+        }
         const bool want = ready && uni_path() && nM == 0;
         if (want == packed) return;
         packed = want;
         graph.reset();          // captured launches carry the layout
-        oneStepAfter.clear();   // and the packed passes move the buffer indices differently
+        oneStepAfter.clear();   // and the packed passes move the shadows' indices differently
         const int n = N();
-        k_sph_pack<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, vel[Vv].p, st[S].p, posq[P].p, velf[Vv].p,
+        k_sph_pack<<<grid_for(n, 256), 256, 0, s>>>(n, pos[P].p, vel[Vv].p, st[S].p, posq[QX].p, velf[QV].p,
                                                     packed ? 1 : 0);
         g_launches += 1;
         DEMSPH_LAUNCH_CHECK();
@@ -2233,7 +2740,7 @@ struct SphScene {
     template <class F>
     void capture_steps(StepGraph& gr, int nsteps, F&& body) {
         if (cond_wanted()) {
-            const std::array<int, 7> idx = {P, Vv, S, R0, D, ID, L};
+            const std::array<int, 9> idx = {P, Vv, S, R0, D, ID, L, QX, QV};
             const bool lists0 = haveLists;
             condCapture = true;
             try {
@@ -2245,6 +2752,7 @@ struct SphScene {
                 condOK = false;
                 (void)cudaGetLastError();
                 P = idx[0]; Vv = idx[1]; S = idx[2]; R0 = idx[3]; D = idx[4]; ID = idx[5]; L = idx[6];
+                QX = idx[7]; QV = idx[8];
                 haveLists = lists0;
             }
         }
@@ -2278,11 +2786,13 @@ struct SphScene {
         SphDev d = dev();
         d.posOut = pos[P ^ 1].p;
         d.velOut = vel[Vv ^ 1].p;
-        d.velfOut = velf[Vv ^ 1].p;
-        d.posqOut = posq[P ^ 1].p;
+        d.velfOut = velf[QV ^ 1].p;
+        d.posqOut = posq[QX ^ 1].p;
+        d.xrOut = xr[QX ^ 1].p;
+        d.vpOut = vp[QV ^ 1].p;
         launch_accel(d, 0.5 * dt, dt, 1, coupling, true);
-        P ^= 1;
-        Vv ^= 1;
+        P ^= 1; QX ^= 1;
+        Vv ^= 1; QV ^= 1;
     }
     // The momentum pass (k_sph_accel) on the state d reads (with the markers'
     // terms when there are markers), preceded inside a coupled step by the
@@ -2291,7 +2801,9 @@ struct SphScene {
     // skin: the first pass of a step on skin lists (first = 1).
     void launch_accel(const SphDev& d, double hdt, double tstep, int first, bool reaction, bool skin = false) {
         const int n = N();
-        const unsigned grid = grid_for(n, kSphPerBlock);
+        const bool wide = n <= kWideFluid && nM == 0;
+        const bool oneWave = n <= device_sms() * 4 * kSphPerBlock;  // every block resident at four per SM
+        const unsigned grid = grid_for(n, kSphPerBlock), ugrid = grid_for(n, kSphBlock / (wide ? kWide : kQuad));
         const bool fp64 = precision == DEMSPH_PRECISION_FP64;
         if (nM > 0) {
             if (reaction) {
@@ -2306,8 +2818,8 @@ struct SphScene {
                 g_launches += 1;
             }
             if (uni_path()) {
-                if (skin) k_sph_accel_u<true, true><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
-                else k_sph_accel_u<false, true><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+                if (skin) k_sph_accel_u<true, true><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+                else k_sph_accel_u<false, true><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
             } else if (skin) {
                 if (fp64) k_sph_accel<double, true, true><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
                 else k_sph_accel<float, true, true><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
@@ -2316,9 +2828,19 @@ struct SphScene {
                 else k_sph_accel<float, true><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
             }
             g_launches += 1;
+        } else if (packed64) {
+            if (wide && skin) k_sph_accel_u64<true, kWide><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else if (wide) k_sph_accel_u64<false, kWide><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else if (oneWave && skin) k_sph_accel_u64<true, kQuad, 4><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else if (oneWave) k_sph_accel_u64<false, kQuad, 4><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else if (skin) k_sph_accel_u64<true><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else k_sph_accel_u64<false><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            g_launches += 1;
         } else if (packed) {
-            if (skin) k_sph_accel_u<true><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
-            else k_sph_accel_u<false><<<grid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            if (wide && skin) k_sph_accel_u<true, false, kWide><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else if (wide) k_sph_accel_u<false, false, kWide><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else if (skin) k_sph_accel_u<true><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
+            else k_sph_accel_u<false><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
             g_launches += 1;
         } else {
             if (skin) {
@@ -2336,36 +2858,46 @@ struct SphScene {
         SphDev d = dev();
         d.posOut = pos[P ^ 1].p;
         d.velOut = vel[Vv ^ 1].p;
-        d.velfOut = velf[Vv ^ 1].p;
-        d.posqOut = posq[P ^ 1].p;
+        d.velfOut = velf[QV ^ 1].p;
+        d.posqOut = posq[QX ^ 1].p;
+        d.xrOut = xr[QX ^ 1].p;
+        d.vpOut = vp[QV ^ 1].p;
         launch_accel(d, 0.5 * dt, dt, first, coupling);
-        if (first) P ^= 1;
-        Vv ^= 1;
+        if (first) { P ^= 1; QX ^= 1; }
+        Vv ^= 1; QV ^= 1;
     }
     void density() {
         SphDev d = dev();
         const int n = N();
         d.stOut = st[S ^ 1].p;
         d.stfOut = stf[S ^ 1].p;
-        const unsigned grid = grid_for(n, kSphPerBlock);
+        const bool wide = n <= kWideFluid && nM == 0;
+        const bool oneWave = n <= device_sms() * 4 * kSphPerBlock;  // every block resident at four per SM
+        const unsigned grid = grid_for(n, kSphPerBlock), ugrid = grid_for(n, kSphBlock / (wide ? kWide : kQuad));
         const bool fp64 = precision == DEMSPH_PRECISION_FP64;
         if (nM > 0) {
-            if (uni_path()) k_sph_density_u<true><<<grid, kSphBlock, 0, s>>>(d, dt);
+            if (uni_path()) k_sph_density_u<true><<<ugrid, kSphBlock, 0, s>>>(d, dt);
             else if (fp64) k_sph_density<double, true><<<grid, kSphBlock, 0, s>>>(d, dt);
             else k_sph_density<float, true><<<grid, kSphBlock, 0, s>>>(d, dt);
             g_launches += 1;
-        } else if (packed) {
-            // the packed shadows carry rho and p: the pass writes the next
-            // buffers of positions and velocities (copies of the records, with
-            // the new rho / p in their shadows) as well
-            d.posOut = pos[P ^ 1].p;
-            d.velOut = vel[Vv ^ 1].p;
-            d.posqOut = posq[P ^ 1].p;
-            d.velfOut = velf[Vv ^ 1].p;
-            k_sph_density_u<false><<<grid, kSphBlock, 0, s>>>(d, dt);
+        } else if (packed64) {
+            // the gathered records carry rho and p: the pass writes their next buffers
+            d.xrOut = xr[QX ^ 1].p;
+            d.vpOut = vp[QV ^ 1].p;
+            if (wide) k_sph_density_u64<kWide><<<ugrid, kSphBlock, 0, s>>>(d, dt);
+            else if (oneWave) k_sph_density_u64<kQuad, 4><<<ugrid, kSphBlock, 0, s>>>(d, dt);
+            else k_sph_density_u64<><<<ugrid, kSphBlock, 0, s>>>(d, dt);
             g_launches += 1;
-            P ^= 1;
-            Vv ^= 1;
+            QX ^= 1;
+            QV ^= 1;
+        } else if (packed) {
+            d.posqOut = posq[QX ^ 1].p;
+            d.velfOut = velf[QV ^ 1].p;
+            if (wide) k_sph_density_u<false, kWide><<<ugrid, kSphBlock, 0, s>>>(d, dt);
+            else k_sph_density_u<false><<<ugrid, kSphBlock, 0, s>>>(d, dt);
+            g_launches += 1;
+            QX ^= 1;
+            QV ^= 1;
         } else {
             if (fp64) k_sph_density<double, false><<<grid, kSphBlock, 0, s>>>(d, dt);
             else k_sph_density<float, false><<<grid, kSphBlock, 0, s>>>(d, dt);
@@ -2394,7 +2926,7 @@ struct SphScene {
     // Two steps per graph: every ping-pong index is back to its parity.
     GraphSet graph;
     bool useGraphs = true;
-    int index_key() const { return P | Vv << 1 | S << 2 | R0 << 3 | D << 4 | ID << 5; }
+    int index_key() const { return P | Vv << 1 | S << 2 | R0 << 3 | D << 4 | ID << 5 | QX << 6 | QV << 7; }
 
     // One step with a CUDA event after every phase, on the scene stream:
     // 0 cell sort, 1 permute + lists, 2 accel + kick + drift, 3 continuity + EOS,
@@ -2587,10 +3119,10 @@ struct SphScene {
             StepGraph& gr = graph.at(key);
             if (!gr.ready()) {
                 capture_steps(gr, 1, [&] { step_body(); });  // moves the host's indices on
-                oneStepAfter[key] = {P, Vv, S, R0, D, ID, L};
+                oneStepAfter[key] = {P, Vv, S, R0, D, ID, L, QX, QV};
             } else {
                 const auto& a = oneStepAfter.at(key);
-                P = a[0]; Vv = a[1]; S = a[2]; R0 = a[3]; D = a[4]; ID = a[5]; L = a[6];
+                P = a[0]; Vv = a[1]; S = a[2]; R0 = a[3]; D = a[4]; ID = a[5]; L = a[6]; QX = a[7]; QV = a[8];
             }
             gr.launch(s);
             iStep += 1;
@@ -2600,7 +3132,7 @@ struct SphScene {
         status_async();
     }
     static constexpr int kOneStepKey = 1 << 10;
-    std::map<int, std::array<int, 7>> oneStepAfter;  // one-step graph key -> indices after the step
+    std::map<int, std::array<int, 9>> oneStepAfter;  // one-step graph key -> indices after the step
 
     // ------------------------------------------------ coupled DEM balls ----
     // Samples balls[0..n) of the DEM scene (radii read from its device
@@ -2727,7 +3259,7 @@ struct SphScene {
                         cgSub = demSub;
                     }
                     for (; k + kCoupledSteps <= n; k += kCoupledSteps) {
-                        StepGraph& gr = cgraph.at(index_key() | dem_graph_key(dem) << 6);
+                        StepGraph& gr = cgraph.at(index_key() | dem_graph_key(dem) << 8);
                         if (!gr.ready()) {
                             const long i0 = iStep;
                             const double t0 = time;
@@ -2894,7 +3426,7 @@ struct SphScene {
             velf[b].alloc(n, s, false); stf[b].alloc(n, s, false); posq[b].alloc(n, s, false);
             rho0[b].alloc(n, s, false); drho[b].alloc(n, s, false); id[b].alloc(n, s, false);
         }
-        P = Vv = S = R0 = D = ID = L = 0;
+        P = Vv = S = R0 = D = ID = L = QX = QV = 0;
         k_iota<<<grid_for(n, 256), 256, 0, s>>>(n, id[0].p);
         g_launches += 1;
         acc.alloc(n, s, true);
@@ -3259,8 +3791,10 @@ int demsph_sph_eval_accel(demsph_sph_t h) {
         SphDev d = s.dev();
         d.posOut = s.pos[s.P ^ 1].p;
         d.velOut = s.vel[s.Vv ^ 1].p;
-        d.velfOut = s.velf[s.Vv ^ 1].p;
-        d.posqOut = s.posq[s.P ^ 1].p;
+        d.velfOut = s.velf[s.QV ^ 1].p;
+        d.posqOut = s.posq[s.QX ^ 1].p;
+        d.xrOut = s.xr[s.QX ^ 1].p;
+        d.vpOut = s.vp[s.QV ^ 1].p;
         s.launch_accel(d, 0.0, 0.0, 0, false);
         DEMSPH_CUDA(cudaStreamSynchronize(s.s));
     });
