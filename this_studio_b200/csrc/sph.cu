@@ -58,6 +58,7 @@ struct UniK {
     float invcD2;  // 1 / c_dummy^2
     float rho0D;   // dummy rest density
     float3 gq;     // gravity times q
+    float h, m, nu;  // the fluid's constants as the unpacked shadows hold them
 };
 
 // The same constants for the FP64 passes (lengths in metres).
@@ -1338,8 +1339,7 @@ __global__ void __launch_bounds__(kSphBlock, kDensityBlocks<R>) k_sph_density(Sp
 
 // ---------------------------------------------------------------------------
 // Mixed-precision passes for scenes with uniform particle constants (UniK);
-// with markers (kMarkers) the shadows stay unpacked and the markers' terms
-// come from the general boundary functions.  Same pair sets, same formulas as
+// with markers (kMarkers) the markers' terms come from the general boundary functions.  Same pair sets, same formulas as
 // k_sph_accel / k_sph_density (updateWCSPHAccelerationKernel and
 // updateWCSPHDensityChangeKernel, WCSPHIntegrationKernel.cu:42-282), with
 // the constants hoisted and the terms regrouped.  With t = max(1 - q_n / 2, 0)
@@ -1449,21 +1449,6 @@ __device__ __forceinline__ OwnU own_u(const SphDev& d, int i) {
     const double4 v = d.vel[i];
     const double4 st = d.st[i];
     return OwnU{d.posq[i], make_float3((float)v.x, (float)v.y, (float)v.z), (float)st.x, (float)st.y};
-}
-// A fluid neighbour's (v, p) and rho: from the packed shadows, or in a scene
-// with markers, whose reaction kernel reads the shadows' usual w components
-// (h, m), from the velocity shadow and the FP32 state (a third gather).
-template <bool kUnpacked>
-__device__ __forceinline__ float4 nb_vp(const SphDev& d, int j, const int4& qj, float& rhoj) {
-    const float4 v = d.velf[j];
-    if constexpr (kUnpacked) {
-        const float4 sj = d.stf[j];
-        rhoj = sj.x;
-        return make_float4(v.x, v.y, v.z, sj.y);
-    } else {
-        rhoj = __int_as_float(qj.w);
-        return v;
-    }
 }
 struct Acc2 {
     float2 x, y, z;
@@ -1662,13 +1647,12 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
         skin_pairs<kLanes>(d.cntV[i], d.nbV, d.KF, i, d.nbF, d.cntF, d.pos, d.g, d.fStart, i,
                    [&](int a, int b, bool two, bool& ka, bool& kb) {
                        const int4 qa = d.posq[a], qb = d.posq[b];
-                       float rhoa, rhob;
-                       const float4 va = nb_vp<kMarkers>(d, a, qa, rhoa), vb = nb_vp<kMarkers>(d, b, qb, rhob);
+                       const float4 va = d.velf[a], vb = d.velf[b];  // (v_j, p_j)
                        PairGeom p = pair_geom(o.q, qa, qb, u);
                        ka = cutoff_u(p.r2.x, u, d.pos, d.pos, i, a);
                        kb = two && cutoff_u(p.r2.y, u, d.pos, d.pos, i, b);
                        p.f = make_float2(ka ? p.f.x : 0.f, kb ? p.f.y : 0.f);
-                       acc_fluid_u(o, p, va, vb, rhoa, rhob, u, acc2);
+                       acc_fluid_u(o, p, va, vb, __int_as_float(qa.w), __int_as_float(qb.w), u, acc2);
                    });
         acc2 = acc2_scaled(acc2, u.aR);
         if (d.ND > 0) {
@@ -1684,11 +1668,10 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
     } else {
         lane_pairs<kLanes>(d.cntF[i], d.nbF, d.KF, i, i, d.pos, d.g, d.fStart, d.pos, [&](int a, int b, bool two) {
             const int4 qa = d.posq[a], qb = d.posq[b];
-            float rhoa, rhob;
-            const float4 va = nb_vp<kMarkers>(d, a, qa, rhoa), vb = nb_vp<kMarkers>(d, b, qb, rhob);
+            const float4 va = d.velf[a], vb = d.velf[b];
             PairGeom p = pair_geom(o.q, qa, qb, u);
             p.f.y = two ? p.f.y : 0.f;
-            acc_fluid_u(o, p, va, vb, rhoa, rhob, u, acc2);
+            acc_fluid_u(o, p, va, vb, __int_as_float(qa.w), __int_as_float(qb.w), u, acc2);
         });
         acc2 = acc2_scaled(acc2, u.aR);
         if (d.ND > 0) {
@@ -1737,11 +1720,11 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
     const double3 v = xyz(vi4) + hdt * a;
     const double4 v4 = d4(v, vi4.w);
     d.velOut[i] = v4;
-    d.velfOut[i] = kMarkers ? f4(v4) : velf_p(v4, s4);
+    d.velfOut[i] = velf_p(v4, s4);
     if (first) {
         const double4 pn = d4(xyz(pi4) + dt * v, pi4.w);
         d.posOut[i] = pn;
-        d.posqOut[i] = kMarkers ? fixq(pn, d.g.mn, d.invq) : fixq_rho(pn, s4, d.g.mn, d.invq);
+        d.posqOut[i] = fixq_rho(pn, s4, d.g.mn, d.invq);
         if constexpr (kSkin) {
             const double3 dd = xyz(pn) - xyz(d.xb[i]);
             atomicMax(d.maxd2 + (blockIdx.x & (kSkinSlots - 1)), __float_as_uint((float)dot(dd, dd)));
@@ -1761,11 +1744,10 @@ __global__ void __launch_bounds__(kSphBlock, 8) k_sph_density_u(SphDev d, double
     float2 sumF = make_float2(0.f, 0.f), sumD = make_float2(0.f, 0.f);
     lane_pairs<kLanes>(d.cntF[i], d.nbF, d.KF, i, i, d.pos, d.g, d.fStart, d.pos, [&](int a, int b, bool two) {
         const int4 qa = d.posq[a], qb = d.posq[b];
-        float rhoa, rhob;
-        const float4 va = nb_vp<kMarkers>(d, a, qa, rhoa), vb = nb_vp<kMarkers>(d, b, qb, rhob);  // (v_j, p_j)
+        const float4 va = d.velf[a], vb = d.velf[b];
         PairGeom p = pair_geom(o.q, qa, qb, u);
         p.f.y = two ? p.f.y : 0.f;
-        add_continuity(o, p, va, vb, make_float2(va.w, vb.w), make_float2(rhoa, rhob), u.dF, sumF);
+        add_continuity(o, p, va, vb, make_float2(va.w, vb.w), make_float2(__int_as_float(qa.w), __int_as_float(qb.w)), u.dF, sumF);
     });
     if (d.ND > 0) {
         lane_pairs<kLanes>(d.cntD[i], d.nbD, d.KD, i, -1, d.pos, d.g, d.dStart, d.dpos, [&](int a, int b, bool two) {
@@ -1798,7 +1780,6 @@ __global__ void __launch_bounds__(kSphBlock, 8) k_sph_density_u(SphDev d, double
     const double4 so = make_double4(ch + r0, s4.z * s4.z * ch, s4.z, s4.w);
     d.stOut[i] = so;
     d.stfOut[i] = f4(so);
-    if constexpr (kMarkers) return;  // unpacked shadows: the state records alone change
     // the packed shadows with the new rho and p
     d.posqOut[i] = make_int4(o.q.x, o.q.y, o.q.z, __float_as_int((float)so.x));
     d.velfOut[i] = make_float4(o.v.x, o.v.y, o.v.z, (float)so.y);
@@ -2023,7 +2004,11 @@ __global__ void k_sph_pack64(int n, const double4* __restrict__ pos, const doubl
 // writes them as this step's transposed rows for the second reaction.
 template <class R>
 constexpr int kMarkerForceBlocks = std::is_same<R, float>::value ? 8 : 4;
-template <class R, bool kSkinRows>
+// kPacked: the fluid's shadows are packed (the specialised passes'), its h, m, c
+// and nu the scene's constants; unpacked, the passes themselves gathered a third
+// record per neighbour (coupled tank of 190,000: first pass 93.2 -> 88.5 us,
+// second 73.8 -> 67.6, continuity 77.6 -> 65.0; the reaction is unchanged).
+template <class R, bool kSkinRows, bool kPacked = false>
 __global__ void __launch_bounds__(kSphBlock, kMarkerForceBlocks<R>) k_sph_marker_force(SphDev d, double w, int add) {
     const int t = blockIdx.x * kSphPerBlock + threadIdx.x / kQuad;
     if (t >= d.NM) return;
@@ -2043,16 +2028,19 @@ __global__ void __launch_bounds__(kSphBlock, kMarkerForceBlocks<R>) k_sph_marker
             // the FP32 shadows hold what fluid_own rounds the FP64 records to;
             // the mass is the shadow's FP32 rounding (relative 6e-8)
             const int4 qa = d.posq[a];
-            const float ha = __int_as_float(qa.w);
+            const float ha = kPacked ? d.uk.h : __int_as_float(qa.w);
             const OwnPos<float> op{mk3(0, 0, 0), qa};
             float3 rij;
             float hj;
             pair_r<float>(op, mv.pos, mv.posq, d.q, t, rij, hj);
             if (test && !cutoff_f(rij, ha, hj, [&] { return d.pos[a]; }, d.mpos, t)) return false;
-            const float4 va = d.velf[a], sa = d.stf[a];
+            const float4 va = d.velf[a];
+            float4 sa;
+            if constexpr (kPacked) sa = make_float4(__int_as_float(qa.w), va.w, d.uk.cF, d.uk.nu);
+            else sa = d.stf[a];
             const FluidOwn<float> o{op, make_float3(va.x, va.y, va.z), sa.x, sa.y, sa.z, sa.w, hconst<float>(ha)};
             boundary_acc_r<R>(d, o, mv, t, rij, hj, g, acc);
-            F -= (double)va.w * up(acc);
+            F -= (double)(kPacked ? d.uk.m : va.w) * up(acc);
         } else {
             const double4 pa = d.pos[a];
             const OwnPos<double> op{xyz(pa), make_int4(0, 0, 0, 0)};
@@ -2320,8 +2308,7 @@ struct SphScene {
         u.on = ok;
         return u;
     }
-    // The uniform-constant passes (mixed precision); with markers they read
-    // the unpacked shadows (packed only when nM == 0).
+    // The uniform-constant passes (mixed precision).
     bool uni_path() const { return uni.on && uniKernels && precision != DEMSPH_PRECISION_FP64; }
     // The FP64 ones serve scenes without markers whose lengths and densities
     // (and their squares) lie well inside the FP32 range: the passes start
@@ -2378,6 +2365,9 @@ struct SphScene {
         k.sD = 0.5 * fix * uni.mD;
         k.c2q = (float)((2.0 * h / qd) * (2.0 * h / qd));
         k.cF = (float)uni.cF;
+        k.h = (float)uni.h;
+        k.m = (float)uni.mF;
+        k.nu = (float)uni.nuF;
         k.cbarD = (float)(0.5 * (uni.cF + uni.cD));
         k.invcD2 = uni.cD > 0 ? (float)(1.0 / (uni.cD * uni.cD)) : 0.0f;
         k.rho0D = (float)uni.rho0D;
@@ -2599,7 +2589,7 @@ struct SphScene {
                 DEMSPH_LAUNCH_CHECK();
             }
         }
-        const bool want = ready && uni_path() && nM == 0;
+        const bool want = ready && uni_path();
         if (want == packed) return;
         packed = want;
         graph.reset();          // captured launches carry the layout
@@ -2810,14 +2800,16 @@ struct SphScene {
                 const unsigned mg = grid_for(nM, kSphPerBlock);
                 if (skin) {
                     if (fp64) k_sph_marker_force<double, true><<<mg, kSphBlock, 0, s>>>(d, 0.5, 0);
+                    else if (packed) k_sph_marker_force<float, true, true><<<mg, kSphBlock, 0, s>>>(d, 0.5, 0);
                     else k_sph_marker_force<float, true><<<mg, kSphBlock, 0, s>>>(d, 0.5, 0);
                 } else {
                     if (fp64) k_sph_marker_force<double, false><<<mg, kSphBlock, 0, s>>>(d, 0.5, first ? 0 : 1);
+                    else if (packed) k_sph_marker_force<float, false, true><<<mg, kSphBlock, 0, s>>>(d, 0.5, first ? 0 : 1);
                     else k_sph_marker_force<float, false><<<mg, kSphBlock, 0, s>>>(d, 0.5, first ? 0 : 1);
                 }
                 g_launches += 1;
             }
-            if (uni_path()) {
+            if (packed) {
                 if (skin) k_sph_accel_u<true, true><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
                 else k_sph_accel_u<false, true><<<ugrid, kSphBlock, 0, s>>>(d, hdt, tstep, first);
             } else if (skin) {
@@ -2876,8 +2868,13 @@ struct SphScene {
         const unsigned grid = grid_for(n, kSphPerBlock), ugrid = grid_for(n, kSphBlock / (wide ? kWide : kQuad));
         const bool fp64 = precision == DEMSPH_PRECISION_FP64;
         if (nM > 0) {
-            if (uni_path()) k_sph_density_u<true><<<ugrid, kSphBlock, 0, s>>>(d, dt);
-            else if (fp64) k_sph_density<double, true><<<grid, kSphBlock, 0, s>>>(d, dt);
+            if (packed) {
+                d.posqOut = posq[QX ^ 1].p;
+                d.velfOut = velf[QV ^ 1].p;
+                k_sph_density_u<true><<<ugrid, kSphBlock, 0, s>>>(d, dt);
+                QX ^= 1;
+                QV ^= 1;
+            } else if (fp64) k_sph_density<double, true><<<grid, kSphBlock, 0, s>>>(d, dt);
             else k_sph_density<float, true><<<grid, kSphBlock, 0, s>>>(d, dt);
             g_launches += 1;
         } else if (packed64) {
@@ -4389,7 +4386,7 @@ int demsph_sph_couple_balls(demsph_sph_t h, demsph_dem_t dem, long n, const int*
         SPH_CHECK(h);
         if (!dem) throw Status(DEMSPH_ERR_INVALID, "null DEM scene handle");
         h->sc.add_bodies(dem, n, balls, spacing, smoothingLength, soundSpeed, viscosity, density);
-        h->sc.sync_mode();  // scenes with markers keep the shadows unpacked
+        h->sc.sync_mode();
     });
 }
 int demsph_sph_couple_step(demsph_sph_t h, demsph_dem_t dem, long n, int demSubsteps) {
