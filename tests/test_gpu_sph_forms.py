@@ -89,3 +89,26 @@ def test_overflowed_rows_are_walked(gpu, prec, n):
         s.setSPH(position=pos)
         s.step(4)
     _same(a.getSPH(), b.getSPH(), 1e-5)
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("width", [0.02, 0.05, 0.2])  # domains from less than one cell to several cells along x
+def test_pair_sets_with_particles_outside_the_domain(gpu, prec, width):
+    """A domain narrower than the fluid: the particles beyond its face are
+    sorted into the last cells, and every pair within the cutoff is found."""
+    sc = _scene(12, 6, 6)
+    minb, maxb = tuple(sc.minb), (sc.minb[0] + width, sc.maxb[1], sc.maxb[2])
+    g = _build(sc, prec, minb=minb, maxb=maxb)
+    g.neighborSearch()
+    cut = 2.0 * 1.3 * sc.spacing
+    for w, other in ((0, sc.fluid), (1, sc.dummy)):
+        d = sc.fluid[:, None] - other[None]
+        near = (d * d).sum(-1) <= cut * cut
+        if w == 0:
+            np.fill_diagonal(near, False)
+        a = pair_keys(*g.getPairs(w))
+        np.testing.assert_array_equal(np.sort(a), np.sort(pair_keys(*np.nonzero(near))))
+    ref = _build(sc, prec, uniform=False, skin=0.0, minb=minb, maxb=maxb)
+    for s in (g, ref):
+        s.step(5)
+    _same(g.getSPH(), ref.getSPH(), TOL[prec])

@@ -125,6 +125,89 @@ static __global__ void k_cell_rank(int n, const int* __restrict__ key, const int
     }
 }
 
+// The whole build of a small table (count, scan, scatter, rank) in one block,
+// the counters in shared memory: the separate kernels' launches are most of a
+// small scene's sort.  1,000 particles: 8.6 -> 1.8 us;
+// 4,096 in 24,576 cells were slower so (16.9 us against 13.2).
+constexpr int kSmallObjs = 2048, kSmallCells = 8192;
+static __global__ void __launch_bounds__(1024) k_cell_small(const double4* __restrict__ p, int n, GridDesc g, int ncell,
+                                                           int* __restrict__ key, int* __restrict__ start,
+                                                           int* __restrict__ unordered, int* __restrict__ sorted,
+                                                           const int* __restrict__ orderKey, int outsideOnly,
+                                                           const int* __restrict__ gate, float4* __restrict__ rec) {
+    if (gate && *gate == 0) return;
+    extern __shared__ int cnt[];
+    __shared__ int warpSums[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    for (int c = t; c < ncell; c += 1024) cnt[c] = 0;
+    __syncthreads();
+    for (int i = t; i < n; i += 1024) {
+        const double4 q = p[i];
+        int k = -1;
+        if (!(outsideOnly && q.x >= g.mn.x && q.x < g.mx.x && q.y >= g.mn.y && q.y < g.mx.y && q.z >= g.mn.z &&
+              q.z < g.mx.z)) {
+            k = clamped_key(mk3(q.x, q.y, q.z), g);
+            atomicAdd(cnt + k, 1);
+        }
+        key[i] = k;
+    }
+    __syncthreads();
+    // exclusive scan, a run of consecutive cells per thread; the counters become
+    // the cells' cursors
+    const int per = (ncell + 1023) / 1024, c0 = min(ncell, t * per), c1 = min(ncell, c0 + per);
+    int s = 0;
+    for (int c = c0; c < c1; c++) s += cnt[c];
+    int x = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) warpSums[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        const int ws = warpSums[lane];
+        int xs = ws;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, xs, o);
+            if (lane >= o) xs += y;
+        }
+        warpSums[lane] = xs - ws;
+        if (lane == 31) start[ncell] = xs;
+    }
+    __syncthreads();
+    int e = x - s + warpSums[w];
+    for (int c = c0; c < c1; c++) {
+        const int m = cnt[c];
+        start[c] = e;
+        cnt[c] = e;
+        e += m;
+    }
+    __syncthreads();
+    for (int i = t; i < n; i += 1024) {
+        const int k = key[i];
+        if (k >= 0) unordered[atomicAdd(cnt + k, 1)] = i;
+    }
+    __syncthreads();  // (the block's own writes to key, start and unordered are visible to it from here)
+    const int total = start[ncell];
+    for (int q = t; q < total; q += 1024) {
+        const int v = unordered[q];
+        const int c = key[v], b = start[c], end = cnt[c];
+        const int kv = orderKey ? orderKey[v] : v;
+        int r = 0;
+        for (int o = b; o < end; o++) {
+            const int u = unordered[o];
+            r += (orderKey ? orderKey[u] : u) < kv;
+        }
+        sorted[b + r] = v;
+        if (rec) {
+            const double4 a = p[v];
+            rec[b + r] = make_float4((float)(a.x - g.mn.x), (float)(a.y - g.mn.y), (float)(a.z - g.mn.z), (float)a.w);
+        }
+    }
+}
+
 // Host side: owns the cell arrays of one grid and builds them on a stream.
 struct CellTable {
     GridDesc g{};
@@ -181,6 +264,13 @@ struct CellTable {
     void build(const double4* p, int n, cudaStream_t s, const int* orderKey = nullptr, bool outsideOnly = false,
                const int* gate = nullptr) {
         launches = 0;
+        if (n > 0 && n <= kSmallObjs && ncell <= kSmallCells) {
+            k_cell_small<<<1, 1024, ncell * sizeof(int), s>>>(p, n, g, ncell, key.p, start.p, unordered.p, sorted.p,
+                                                              orderKey, outsideOnly ? 1 : 0, gate, rec.p);
+            launches = 1;
+            DEMSPH_LAUNCH_CHECK();
+            return;
+        }
         if (n > 0) {
             k_cell_count<<<grid_for(n, 256), 256, 0, s>>>(p, n, g, key.p, cnt.p, outsideOnly ? 1 : 0, gate);
             launches++;

@@ -572,9 +572,12 @@ static constexpr double kPi = 3.14159265358979323846;
 // ----------------------------------------------------------------- grid ---
 // spatialGrid (DEMSPH/kernel/boundary.h:70-94): cells of at least the
 // requested size tiling [mn, mx); keys z*ny*nx + y*nx + x.
+// A grid may be refined along x (grid_refine_x): cells a fraction of the
+// requested size wide, rx of them to the requested reach.
 struct GridDesc {
     double3 mn, mx, cs;
     int nx, ny, nz;
+    int rx = 1;  // cells along x that cover the requested size
     int ncell() const { return nx * ny * nz; }
 };
 static inline bool grid_set(GridDesc& g, double3 mn, double3 mx, double cell) {
@@ -587,6 +590,14 @@ static inline bool grid_set(GridDesc& g, double3 mn, double3 mx, double cell) {
     g.nz = d.z > cell ? int(d.z / cell) : 1;
     g.cs = mk3(d.x / double(g.nx), d.y / double(g.ny), d.z / double(g.nz));
     return true;
+}
+// Splits every cell into k along x.  Objects sorted into the finer cells lie
+// in x order along a row of cells, so the neighbours of an object within a
+// stencil row are nearly consecutive in memory.
+static inline void grid_refine_x(GridDesc& g, int k) {
+    g.nx *= k;
+    g.cs.x = (g.mx.x - g.mn.x) / double(g.nx);
+    g.rx *= k;
 }
 // calculateGridPosition (neighborSearchKernel.cuh:4-9): truncation toward zero.
 __host__ __device__ __forceinline__ int3 cell_of(double3 p, const GridDesc& g) {
@@ -626,12 +637,25 @@ __device__ __forceinline__ Stencil stencil_of_cell3(int3 c, const GridDesc& g) {
     st.c = c;
     st.s = make_int3(-1, -1, -1);
     st.e = make_int3(1, 1, 1);
-    if (st.c.x <= 0) { st.c.x = 0; st.s.x = 0; }
-    if (st.c.x >= g.nx - 1) { st.c.x = g.nx - 1; st.e.x = 0; }
-    if (st.c.y <= 0) { st.c.y = 0; st.s.y = 0; }
-    if (st.c.y >= g.ny - 1) { st.c.y = g.ny - 1; st.e.y = 0; }
-    if (st.c.z <= 0) { st.c.z = 0; st.s.z = 0; }
-    if (st.c.z >= g.nz - 1) { st.c.z = g.nz - 1; st.e.z = 0; }
+    st.c.x = min(max(st.c.x, 0), g.nx - 1);
+    st.s.x = max(-g.rx, -st.c.x);
+    st.e.x = min(g.rx, g.nx - 1 - st.c.x);
+    // (clamped first: beyond the face of a domain one cell wide, the reference's
+    // two clamps in turn leave a row before the table's first)
+    st.c.y = min(max(st.c.y, 0), g.ny - 1);
+    st.c.z = min(max(st.c.z, 0), g.nz - 1);
+    if (st.c.y == 0) st.s.y = 0;
+    if (st.c.y == g.ny - 1) st.e.y = 0;
+    if (st.c.z == 0) st.s.z = 0;
+    if (st.c.z == g.nz - 1) st.e.z = 0;
+    return st;
+}
+// The common stencil of a group of rx cells along x (one cell of the unrefined
+// grid): group k holds the cells [k rx, (k + 1) rx).
+__device__ __forceinline__ Stencil stencil_of_group(int k, const GridDesc& g) {
+    const int n = g.nx / g.rx;
+    Stencil st = stencil_of_cell3(make_int3(k % n * g.rx, (k / n) % g.ny, k / (n * g.ny)), g);
+    st.e.x = min(2 * g.rx - 1, g.nx - 1 - st.c.x);
     return st;
 }
 // Calls f(begin, end) for each stencil row range of the sorted list.

@@ -76,6 +76,7 @@ struct SphDev {
     int N, ND, KF, KD;
     GridDesc g;
     const int* fStart;   // fluid cell start (new order)
+    const int* fGroups;  // the groups of rx cells that hold fluid: their count, then their numbers
     const int* dStart;   // dummy cell start (dummies stored in cell order)
     const double4* pos;  // current fluid pos
     const double4* lpos; // fluid pos when this step's lists were built (same slot order)
@@ -388,7 +389,8 @@ struct SkinState {
 // IF node around the rebuild (setCond = 1), so a step that keeps its lists
 // launches none of the rebuild's kernels.
 __global__ void __launch_bounds__(kSkinSlots) k_sph_skin_decide(SkinState* st, float half2,
-                                                                 cudaGraphConditionalHandle cond, int setCond) {
+                                                                 cudaGraphConditionalHandle cond, int setCond,
+                                                                 int* groups) {
     __shared__ unsigned m[kSkinSlots];
     const int t = threadIdx.x;
     m[t] = st->maxd2[t];
@@ -405,6 +407,7 @@ __global__ void __launch_bounds__(kSkinSlots) k_sph_skin_decide(SkinState* st, f
         if (r) {
             st->force = 0;
             st->rebuilds++;
+            groups[0] = 0;
         }
         if (setCond) cudaGraphSetConditional(cond, r ? 1u : 0u);
     }
@@ -585,10 +588,13 @@ __global__ void k_sph_permute(int n, const int* __restrict__ sorted, const doubl
                               int* __restrict__ id2, float4* __restrict__ posf, float4* __restrict__ velf2,
                               float4* __restrict__ stf2, int4* __restrict__ posq2, double3 origin, double invq,
                               const int* __restrict__ gate, int packed, double4* __restrict__ xr2,
-                              double4* __restrict__ vp2) {
+                              double4* __restrict__ vp2, const int* __restrict__ key, const int* __restrict__ start,
+                              int rx, int* __restrict__ groups) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n || (gate && *gate == 0)) return;
     int o = sorted[t];
+    const int g = key[o] / rx;
+    if (start[g * rx] == t) groups[1 + atomicAdd(groups, 1)] = g;  // the first of its group
     double4 p = pos[o];
     pos2[t] = p;
     const double4 v = vel[o], q = st[o];
@@ -611,9 +617,11 @@ __global__ void k_sph_permute(int n, const int* __restrict__ sorted, const doubl
 // kernels (SPHNeighborSearchKernel.cu:6-228) in one pass: j != i,
 // |r_ij| <= 2 max(h_i, h_j), rows in the reference's stencil order.
 //
-// Built one warp per cell (the warps stride over the cells with a grid of a
-// few blocks per SM, so that a launch gated off by the skin decision, or the
-// empty cells of a mostly empty domain, cost little).  All particles of a
+// Built one warp per cell that holds fluid -- per group of the finer cells the
+// particles are sorted by, which make up a cell; the reorder lists the groups,
+// so that no warp of a block idles on the empty cells of the air -- (the warps
+// stride over the groups with a grid of a few blocks per SM, so that a launch
+// gated off by the skin decision costs little).  All particles of a
 // cell share the cell's 27-cell stencil (the reference clamps positions and
 // cell indices the same way for
 // every particle of a cell), so the warp stages the stencil's candidates --
@@ -794,21 +802,255 @@ __device__ __forceinline__ void cell_lists(int ps, int pe, const Stencil& st, co
     }
 }
 
+// cell_lists for skin rows of one common h (what a fluid step rebuilds): four
+// own particles share each staged load, their distances in packed FP32 (the
+// stage holds the candidates' negated coordinates), and there is no band: a
+// skin row only has to hold every pair within the cutoff, so the widened FP32
+// test alone decides.  Bound by instruction issue; a
+// dam break of 128,000: 45.4 -> 36.8 us, of a million 227 -> 178, in the groups'
+// order below.
+template <int kStage>
+__device__ __forceinline__ void cell_skin_rows(int ps, int pe, const Stencil& st, const GridDesc& g,
+                                               const int* __restrict__ cellStart, const float4* __restrict__ ownf,
+                                               const float4* __restrict__ otherf, float hi, bool same, int K,
+                                               int* __restrict__ nb, int* __restrict__ cnt, int* needMax, int* overflow,
+                                               float4* __restrict__ stage) {
+    constexpr int kOwn = 4;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    int total = 0;
+    for_stencil_rows(st, g, cellStart, [&](int b, int e) { total += e - b; });
+    if (total == 0) {
+        for (int i = ps + lane; i < pe; i += 32) cnt[i] = 0;
+        return;
+    }
+    const int nchunk = (total + kStage - 1) / kStage;
+    for (int ch = 0; ch < nchunk; ch++) {
+        const int c0 = ch * kStage, c1 = min(total, c0 + kStage);
+        const int m = c1 - c0, mp = (m + 31) & ~31;
+        __syncwarp();
+        int off = 0;
+        for_stencil_rows(st, g, cellStart, [&](int b, int e) {
+            const int lo = max(b, b + (c0 - off)), end = min(e, b + (c1 - off));
+            for (int j = lo + lane; j < end; j += 32) {
+                const float4 q = otherf[j];
+                stage[off + (j - b) - c0] = make_float4(-q.x, -q.y, -q.z, __int_as_float(j));
+            }
+            off += e - b;
+        });
+        if (m + lane < mp) stage[m + lane] = make_float4(1.0e18f, 1.0e18f, 1.0e18f, __int_as_float(-1));
+        __syncwarp();
+        for (int i0 = ps; i0 < pe; i0 += kOwn) {
+            float4 p[kOwn];
+            int n[kOwn];
+            int* row[kOwn];
+#pragma unroll
+            for (int k = 0; k < kOwn; k++) {
+                const int i = min(i0 + k, pe - 1);  // (a missing one repeats the last; its row is not written)
+                p[k] = ownf[i];
+                n[k] = ch == 0 ? 0 : cnt[i];
+                row[k] = nb + row_base(i, K);
+            }
+            for (int v0 = 0; v0 < mp; v0 += 32) {
+                const float4 q = stage[v0 + lane];
+                const int j = __float_as_int(q.w);
+                bool in[kOwn];
+#pragma unroll
+                for (int k = 0; k < kOwn; k += 2) {
+                    const float2 dx = __fadd2_rn(make_float2(p[k].x, p[k + 1].x), make_float2(q.x, q.x));
+                    const float2 dy = __fadd2_rn(make_float2(p[k].y, p[k + 1].y), make_float2(q.y, q.y));
+                    const float2 dz = __fadd2_rn(make_float2(p[k].z, p[k + 1].z), make_float2(q.z, q.z));
+                    const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                    in[k] = d2.x <= hi;
+                    in[k + 1] = d2.y <= hi;
+                }
+                if (same) {
+#pragma unroll
+                    for (int k = 0; k < kOwn; k++) in[k] = in[k] && j != i0 + k;
+                }
+#pragma unroll
+                for (int k = 0; k < kOwn; k++) {
+                    const unsigned h = __ballot_sync(0xffffffffu, in[k]);
+                    if (h == 0) continue;
+                    const int at = n[k] + __popc(h & lt);
+                    if (in[k] && at < K && i0 + k < pe) row[k][at + 28 * (at >> 2)] = j;
+                    n[k] += __popc(h);
+                }
+            }
+            if (lane < kOwn && i0 + lane < pe) {
+                const int c = lane == 0 ? n[0] : lane == 1 ? n[1] : lane == 2 ? n[2] : n[3];
+                const int i = i0 + lane;
+                if (ch + 1 < nchunk) {
+                    cnt[i] = c;
+                } else if (c > K) {  // the passes walk this particle's stencil instead
+                    atomicMax(needMax, c);
+                    atomicExch(overflow, 1);
+                    cnt[i] = -1;
+                } else {
+                    cnt[i] = c;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// The same rows with one own particle per lane, where a warp has a whole cell
+// (some twenty particles): a candidate pair is one broadcast read and six packed
+// operations for all of them, a hit one byte in the lane's column of shared
+// memory, and the rows go out a 128-byte line at a time (the lines of the row
+// layout: 4 entries of 8 consecutive objects).  Candidates are staged kRowStage
+// at a time, so a column never outgrows kRowStage entries.  Half the
+// instructions of the candidate-per-lane form above (ballots and scattered
+// stores); 128,000: 36.8 -> 31.0 us, a million 178 -> 150.
+constexpr int kRowStage = 128;
+constexpr int kRowWords = kRowStage + kRowStage * 32 / 16;  // float4 of shared memory per warp: stage, columns
+__device__ __forceinline__ void cell_rows_by_lane(int ps, int pe, const Stencil& st, const GridDesc& g,
+                                                  const int* __restrict__ cellStart, const float4* __restrict__ ownf,
+                                                  const float4* __restrict__ otherf, float hi, bool same, int K,
+                                                  int* __restrict__ nb, int* __restrict__ cnt, int* needMax,
+                                                  int* overflow, float4* __restrict__ shared) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const float4* __restrict__ pairs = shared;  // (-x0, -x1, -y0, -y1), (-z0, -z1, j0, j1) of two candidates
+    float* __restrict__ stage = reinterpret_cast<float*>(shared);
+    unsigned char* __restrict__ column = reinterpret_cast<unsigned char*>(shared + kRowStage) + lane;
+    const unsigned char* __restrict__ columns = reinterpret_cast<unsigned char*>(shared + kRowStage);
+    // stencil row r: its first candidate and its place among all candidates
+    int b = 0, len = 0;
+    if (lane < 9) {
+        const int zz = lane / 3 - 1, yy = lane % 3 - 1;
+        if (zz >= st.s.z && zz <= st.e.z && yy >= st.s.y && yy <= st.e.y) {
+            const int k = key_of(make_int3(st.c.x, st.c.y + yy, st.c.z + zz), g);
+            b = __ldg(cellStart + k + st.s.x);
+            len = __ldg(cellStart + k + st.e.x + 1) - b;
+        }
+    }
+    int off = len;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const int v = __shfl_up_sync(kAll, off, o);
+        if (lane >= o) off += v;
+    }
+    const int total = __shfl_sync(kAll, off, 8);
+    off -= len;
+    int first[9], shift[9];
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        first[r] = __shfl_sync(kAll, off, r);
+        shift[r] = __shfl_sync(kAll, b - off, r);
+    }
+    const int K4 = (K + 3) & ~3;
+    for (int s0 = ps; s0 < pe; s0 += 32) {
+        const int i = s0 + lane, s1 = min(s0 + 32, pe);
+        const bool has = i < pe;
+        const float4 p = has ? ownf[i] : make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.0f);
+        const float2 px = make_float2(p.x, p.x), py = make_float2(p.y, p.y), pz = make_float2(p.z, p.z);
+        int n = 0;
+        for (int c0 = 0; c0 < total; c0 += kRowStage) {
+            const int m = min(kRowStage, total - c0);
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < kRowStage; u += 32) {
+                const int v = u + lane, c = c0 + v;
+                float4 q = make_float4(-1.0e18f, 0.0f, 0.0f, 0.0f);
+                int j = -1;
+                if (v < m) {
+                    int sh = shift[0];
+#pragma unroll
+                    for (int r = 1; r < 9; r++) sh = c >= first[r] ? shift[r] : sh;
+                    j = c + sh;
+                    q = otherf[j];
+                }
+                float* w = stage + 8 * (v >> 1) + (v & 1);
+                w[0] = -q.x;
+                w[2] = -q.y;
+                w[4] = -q.z;
+                w[6] = __int_as_float(j);
+            }
+            __syncwarp();
+            unsigned char* w = column;
+#pragma unroll 4
+            for (int v = 0; v < m; v += 2) {
+                const float4 a = pairs[v], q = pairs[v + 1];
+                const float2 dx = __fadd2_rn(px, make_float2(a.x, a.y));
+                const float2 dy = __fadd2_rn(py, make_float2(a.z, a.w));
+                const float2 dz = __fadd2_rn(pz, make_float2(q.x, q.y));
+                const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                bool in0 = d2.x <= hi, in1 = d2.y <= hi;
+                if (same) {
+                    in0 = in0 && __float_as_int(q.z) != i;
+                    in1 = in1 && __float_as_int(q.w) != i;
+                }
+                if (in0) { *w = (unsigned char)v; w += 32; }
+                if (in1) { *w = (unsigned char)(v + 1); w += 32; }
+            }
+            const int n1 = n + (int)(w - column) / 32;
+            __syncwarp();
+            for (int blk = s0 >> 3; blk <= (s1 - 1) >> 3; blk++) {
+                const int src = blk * 8 + (lane >> 2) - s0;
+                const bool own = src >= 0 && src < s1 - s0;
+                const int o0 = __shfl_sync(kAll, n, src & 31), o1 = __shfl_sync(kAll, n1, src & 31);
+                const int end = own ? min(o1, K) : 0;
+                const int lo = (int)__reduce_min_sync(kAll, own ? (unsigned)o0 : 0xffffu) >> 2;
+                const int top = ((int)__reduce_max_sync(kAll, (unsigned)end) + 3) >> 2;
+                int* __restrict__ row = nb + (size_t)blk * K4 * 8 + lane;
+                for (int l = lo; l < top; l++) {
+                    const int k = 4 * l + (lane & 3);
+                    if (k >= o0 && k < end) {
+                        const int v = columns[(k - o0) * 32 + src];
+                        row[32 * l] = __float_as_int(stage[8 * (v >> 1) + 6 + (v & 1)]);
+                    }
+                }
+            }
+            n = n1;
+        }
+        if (has) {
+            if (n > K) {  // the passes walk this particle's stencil instead
+                atomicMax(needMax, n);
+                atomicExch(overflow, 1);
+                n = -1;
+            }
+            cnt[i] = n;
+        }
+    }
+}
+
 template <bool kUniformH, int kShape, bool kMarkers>
 __global__ void __launch_bounds__(32 * kListShapes[kShape].warps, kListShapes[kShape].minBlocks)
-    k_sph_lists_cell(SphDev d, int ncell) {
+    k_sph_lists_cell(SphDev d, int parts) {
     constexpr int kListWarps = kListShapes[kShape].warps, kStage = kListShapes[kShape].stage;
     __shared__ float4 sPos[kListWarps][kStage];
     __shared__ int sIdx[kUniformH ? 1 : kListWarps][kUniformH ? 1 : kStage];
     const int w = threadIdx.x >> 5;
     if (d.gate && *d.gate == 0) return;
     ListStage<kUniformH> sg{sPos[w], kUniformH ? nullptr : sIdx[kUniformH ? 0 : w]};
-    for (int cell = blockIdx.x * kListWarps + w; cell < ncell; cell += gridDim.x * kListWarps) {
-        const int ps = d.fStart[cell], pe = d.fStart[cell + 1];
+    const int groups = d.fGroups[0];
+    for (int at = blockIdx.x * kListWarps + w; at < groups * parts; at += gridDim.x * kListWarps) {
+        const int cell = d.fGroups[1 + at / parts], part = at % parts;
+        const int cs = d.fStart[cell * d.g.rx], len = d.fStart[(cell + 1) * d.g.rx] - cs;
+        const int ps = cs + len * part / parts, pe = cs + len * (part + 1) / parts;
         if (ps == pe) continue;
-        // stencil of the cell: the one every particle of the cell computes
         const double4 p0 = d.pos[ps];
-        Stencil st = stencil_of(xyz(p0), d.g);
+        const Stencil st = stencil_of_group(cell, d.g);
+        if constexpr (kUniformH && !kMarkers) {
+            if (d.skin > 0.0f) {
+                const float cut = 2.0f * (float)p0.w + d.skin;
+                const float hi = cut * cut + list_band(cut, d.eps);
+                if (kStage >= kRowWords && parts == 1) {
+                    cell_rows_by_lane(ps, pe, st, d.g, d.fStart, d.posf, d.posf, hi, true, d.KF, d.nbF, d.cntF,
+                                      &d.status->need_pairs, &d.status->overflow, sPos[w]);
+                    cell_rows_by_lane(ps, pe, st, d.g, d.dStart, d.posf, d.dposf, hi, false, d.KD, d.nbD, d.cntD,
+                                      &d.status->need_aux, &d.status->overflow, sPos[w]);
+                } else {
+                    cell_skin_rows<kStage>(ps, pe, st, d.g, d.fStart, d.posf, d.posf, hi, true, d.KF, d.nbF, d.cntF,
+                                           &d.status->need_pairs, &d.status->overflow, sPos[w]);
+                    cell_skin_rows<kStage>(ps, pe, st, d.g, d.dStart, d.posf, d.dposf, hi, false, d.KD, d.nbD, d.cntD,
+                                           &d.status->need_aux, &d.status->overflow, sPos[w]);
+                }
+                continue;
+            }
+        }
         cell_lists<kUniformH, kStage>(ps, pe, st, d.g, d.fStart, d.pos, d.posf, d.pos, d.posf, d.eps, true, d.KF, d.N,
                                       d.nbF, d.cntF, &d.status->need_pairs, &d.status->overflow, sg, d.skin);
         if (d.ND > 0)
@@ -838,9 +1080,9 @@ __global__ void __launch_bounds__(32 * kListShapes[kShape].warps, kListShapes[kS
     if (d.gate && *d.gate == 0) return;
     ListStage<kUniformH> sg{sPos[w], kUniformH ? nullptr : sIdx[kUniformH ? 0 : w]};
     for (int cell = blockIdx.x * kListWarps + w; cell < ncell; cell += gridDim.x * kListWarps) {
-        const int ps = d.mStart[cell], pe = d.mStart[cell + 1];
+        const int ps = d.mStart[cell * d.g.rx], pe = d.mStart[(cell + 1) * d.g.rx];
         if (ps == pe) continue;
-        Stencil st = stencil_of(xyz(d.mpos[ps]), d.g);
+        const Stencil st = stencil_of_group(cell, d.g);
         cell_lists<kUniformH, kStage>(ps, pe, st, d.g, d.fStart, d.mpos, d.mposf, d.pos, d.posf, d.eps, false, d.KR,
                                       d.NM, d.nbR, d.cntR, &d.status->need_mrev, &d.status->overflow, sg, d.skin);
     }
@@ -850,17 +1092,19 @@ __global__ void __launch_bounds__(32 * kListShapes[kShape].warps, kListShapes[kS
 // rebuild (gated), within the cutoff plus the skin.
 template <bool kUniformH, int kShape>
 __global__ void __launch_bounds__(32 * kListShapes[kShape].warps, kListShapes[kShape].minBlocks)
-    k_sph_marker_rows(SphDev d, int ncell) {
+    k_sph_marker_rows(SphDev d) {
     constexpr int kListWarps = kListShapes[kShape].warps, kStage = kListShapes[kShape].stage;
     __shared__ float4 sPos[kListWarps][kStage];
     __shared__ int sIdx[kUniformH ? 1 : kListWarps][kUniformH ? 1 : kStage];
     const int w = threadIdx.x >> 5;
     if (d.gate && *d.gate == 0) return;
     ListStage<kUniformH> sg{sPos[w], kUniformH ? nullptr : sIdx[kUniformH ? 0 : w]};
-    for (int cell = blockIdx.x * kListWarps + w; cell < ncell; cell += gridDim.x * kListWarps) {
-        const int ps = d.fStart[cell], pe = d.fStart[cell + 1];
+    const int groups = d.fGroups[0];
+    for (int at = blockIdx.x * kListWarps + w; at < groups; at += gridDim.x * kListWarps) {
+        const int cell = d.fGroups[1 + at];
+        const int ps = d.fStart[cell * d.g.rx], pe = d.fStart[(cell + 1) * d.g.rx];
         if (ps == pe) continue;
-        Stencil st = stencil_of_cell(cell, d.g);
+        const Stencil st = stencil_of_group(cell, d.g);
         cell_lists<kUniformH, kStage>(ps, pe, st, d.g, d.mStart, d.pos, d.posf, d.mpos, d.mposf, d.eps, false, d.KM,
                                       d.N, d.nbM, d.cntM, &d.status->need_mark, &d.status->overflow, sg, d.skin);
     }
@@ -2229,6 +2473,9 @@ struct SphScene {
     int KF = 96, KD = 64, KDD = 96;
     double listHeadroom = 0.125;  // row capacity above the initial longest row (autotuner)
     CellTable fCells, dCells;
+    DBuf<int> fGroups;
+    static constexpr int kFineX = 4;                      // the sort's cells per grid cell along x
+    static constexpr long long kMaxFineCells = 1LL << 25;  // (a larger, mostly empty domain keeps plain cells)
     DBuf<double4> pos[2], vel[2], st[2];
     DBuf<double> rho0[2], drho[2];
     DBuf<int> id[2];
@@ -2408,6 +2655,7 @@ struct SphScene {
         d.N = N(); d.ND = ND(); d.KF = KF; d.KD = KD;
         d.g = fCells.g;
         d.fStart = fCells.start.p;
+        d.fGroups = fGroups.p;
         d.dStart = dCells.start.p;
         d.pos = pos[P].p; d.lpos = pos[L].p; d.vel = vel[Vv].p; d.st = st[S].p; d.rho0 = rho0[R0].p; d.drho = drho[D].p;
         d.acc = acc.p;
@@ -2485,18 +2733,23 @@ struct SphScene {
     template <int S>
     void launch_lists_shape(const SphDev& d, bool withMarkers) {
         constexpr int W = kListShapes[S].warps;
-        const unsigned grid = list_grid<S>(fCells.ncell);
+        // a small fluid's cells are fewer than the warps the GPU holds: several
+        // warps then share a cell's particles (some twenty), each staging the
+        // cell's candidates for its share.  1,000 particles: 7.8 -> 3.9 us.
+        const int parts = std::min(8, std::max(1, 70000 / std::max(1, N())));
+        const int ncoarse = fCells.ncell / fCells.g.rx;
+        const unsigned grid = list_grid<S>(std::min(ncoarse, N()) * parts);
         if (withMarkers && nM > 0) {
-            if (uniformH) k_sph_lists_cell<true, S, true><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
-            else k_sph_lists_cell<false, S, true><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
+            if (uniformH) k_sph_lists_cell<true, S, true><<<grid, 32 * W, 0, s>>>(d, parts);
+            else k_sph_lists_cell<false, S, true><<<grid, 32 * W, 0, s>>>(d, parts);
             if (coupling) {  // the transposed rows the reaction reads
-                if (uniformH) k_sph_marker_lists<true, S><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
-                else k_sph_marker_lists<false, S><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
+                if (uniformH) k_sph_marker_lists<true, S><<<grid, 32 * W, 0, s>>>(d, ncoarse);
+                else k_sph_marker_lists<false, S><<<grid, 32 * W, 0, s>>>(d, ncoarse);
                 g_launches += 1;
             }
         } else {
-            if (uniformH) k_sph_lists_cell<true, S, false><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
-            else k_sph_lists_cell<false, S, false><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
+            if (uniformH) k_sph_lists_cell<true, S, false><<<grid, 32 * W, 0, s>>>(d, parts);
+            else k_sph_lists_cell<false, S, false><<<grid, 32 * W, 0, s>>>(d, parts);
         }
     }
     // withMarkers: the fluid-marker rows (and, inside a coupled step, the
@@ -2514,12 +2767,13 @@ struct SphScene {
     template <int S>
     void launch_marker_rows_shape(const SphDev& d) {
         constexpr int W = kListShapes[S].warps;
-        const unsigned grid = list_grid<S>(fCells.ncell);
-        if (uniformH) k_sph_marker_rows<true, S><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
-        else k_sph_marker_rows<false, S><<<grid, 32 * W, 0, s>>>(d, fCells.ncell);
-        const unsigned mgrid = list_grid<S>(mCells.ncell);
-        if (uniformH) k_sph_marker_lists<true, S><<<mgrid, 32 * W, 0, s>>>(d, mCells.ncell);
-        else k_sph_marker_lists<false, S><<<mgrid, 32 * W, 0, s>>>(d, mCells.ncell);
+        const int ncoarse = fCells.ncell / fCells.g.rx;
+        const unsigned grid = list_grid<S>(std::min(ncoarse, N()));
+        if (uniformH) k_sph_marker_rows<true, S><<<grid, 32 * W, 0, s>>>(d);
+        else k_sph_marker_rows<false, S><<<grid, 32 * W, 0, s>>>(d);
+        const unsigned mgrid = list_grid<S>(ncoarse);  // (the markers' cells)
+        if (uniformH) k_sph_marker_lists<true, S><<<mgrid, 32 * W, 0, s>>>(d, ncoarse);
+        else k_sph_marker_lists<false, S><<<mgrid, 32 * W, 0, s>>>(d, ncoarse);
         g_launches += 2;
     }
     void launch_marker_rows(const SphDev& d) {
@@ -2533,12 +2787,17 @@ struct SphScene {
     // Moves the fluid records (and their FP32 shadows) into this step's cell order.
     void permute(const int* gate = nullptr) {
         const int n = N();
+        if (!gate) {  // (with a gate the decision that opens it empties the group list)
+            k_zero_ints<<<1, 32, 0, s>>>(fGroups.p, 1);
+            g_launches += 1;
+        }
         k_sph_permute<<<grid_for(n, 256), 256, 0, s>>>(n, fCells.sorted.p, pos[P].p, vel[Vv].p, st[S].p, rho0[R0].p,
                                                        drho[D].p, id[ID].p, pos[P ^ 1].p, vel[Vv ^ 1].p, st[S ^ 1].p,
                                                        rho0[R0 ^ 1].p, drho[D ^ 1].p, id[ID ^ 1].p, posf.p,
                                                        velf[QV ^ 1].p, stf[S ^ 1].p, posq[QX ^ 1].p, fCells.g.mn,
                                                        invq, gate, packed ? 1 : 0, packed64 ? xr[QX ^ 1].p : nullptr,
-                                                       packed64 ? vp[QV ^ 1].p : nullptr);
+                                                       packed64 ? vp[QV ^ 1].p : nullptr, fCells.key.p, fCells.start.p, fCells.g.rx,
+                                                       fGroups.p);
         if (gate) {  // a device-side decision: copy back instead of flipping the indices
             k_sph_copy_back<<<grid_for(n, 256), 256, 0, s>>>(
                 n, gate, pos[P ^ 1].p, vel[Vv ^ 1].p, st[S ^ 1].p, rho0[R0 ^ 1].p, drho[D ^ 1].p, id[ID ^ 1].p,
@@ -2653,7 +2912,7 @@ struct SphScene {
         const bool move = coupling && nM > 0;
         if (move) marker_place(true);
         k_sph_skin_decide<<<1, kSkinSlots, 0, s>>>(skinState.p, (float)(0.25 * skin_abs() * skin_abs()),
-                                                   cudaGraphConditionalHandle(), 0);
+                                                   cudaGraphConditionalHandle(), 0, fGroups.p);
         if (move) marker_sort(gate);
         fCells.build(pos[P].p, N(), s, id[ID].p, false, gate);
         g_launches += 1 + fCells.launches;
@@ -2687,7 +2946,7 @@ struct SphScene {
         DEMSPH_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
         cudaGraphConditionalHandle h;
         DEMSPH_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-        k_sph_skin_decide<<<1, kSkinSlots, 0, s>>>(skinState.p, (float)(0.25 * skin_abs() * skin_abs()), h, 1);
+        k_sph_skin_decide<<<1, kSkinSlots, 0, s>>>(skinState.p, (float)(0.25 * skin_abs() * skin_abs()), h, 1, fGroups.p);
         g_launches += 1;
         DEMSPH_LAUNCH_CHECK();
         DEMSPH_CUDA(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
@@ -3144,7 +3403,7 @@ struct SphScene {
         if (!(dx > 0) || !(hm > 0) || !(c > 0) || !(rho0 > 0) || !(nu >= 0))
             throw Status(DEMSPH_ERR_INVALID, "marker spacing, h, sound speed and density must be positive");
         const GridDesc& g = fCells.g;
-        if (2.0 * hm > std::min(g.cs.x, std::min(g.cs.y, g.cs.z)) * (1.0 + 1e-12))
+        if (2.0 * hm > std::min(g.cs.x * g.rx, std::min(g.cs.y, g.cs.z)) * (1.0 + 1e-12))
             throw Status(DEMSPH_ERR_INVALID, "marker h above the fluid's largest h");
         const DemBodies B = dem_bodies(dem);
         std::vector<double4> bp(B.n);
@@ -3414,9 +3673,15 @@ struct SphScene {
         const double cell = 2.0 * hmax * (1.0 + skinMax) * cellFactor;
         GridDesc gd{};
         if (!grid_set(gd, mn, mx, cell)) throw Status(DEMSPH_ERR_SCENE, "invalid domain or cell size");
+        // Finer cells along x leave a cell's particles in x order: the rows of
+        // neighbouring particles then name runs of consecutive particles.  18,000
+        // in FP64 73.2 -> 70.0 us a step, eight tanks of a batch 178.8 -> 176.4,
+        // larger fluids within 0.5% (passes 1-2% shorter, list build 8% longer).
+        if ((long long)gd.nx * gd.ny * gd.nz * kFineX <= kMaxFineCells) grid_refine_x(gd, kFineX);
         status.alloc(1, s, true);
         const int n = N(), nd = ND();
         fCells.setup(gd, n, s);
+        fGroups.alloc((size_t)n + 1, s, true);
         dCells.setup(gd, std::max(nd, 1), s);
         for (int b = 0; b < 2; b++) {
             pos[b].alloc(n, s, false); vel[b].alloc(n, s, false); st[b].alloc(n, s, false);
