@@ -107,6 +107,12 @@ struct DemDev {
     const int4* tris;
     double4* tcenter;
     const int* triOrder;
+    // the triangles in table order: vertices, and (cell key, triangle, wall, wall
+    // material), so that a ball reads a candidate with one step of loads
+    double4* trA;
+    double4* trB;
+    double4* trC;
+    int4* trI;
     const int* triKey;
     const int* triCellStart;
     double4* wbox;  // [min, max] corners of the mesh vertices' box
@@ -170,13 +176,11 @@ __device__ __forceinline__ void record_pair(const DemDev& d, int slot, int A, in
 // (lane 0 the ninth as well) and a prefix over the lanes restores the row
 // order.  kLanes = 1: one thread per ball with the next row's bounds loaded
 // ahead and four candidates in flight.  Candidates are read as the sort's
-// cell-ordered FP32 records, 16 contiguous bytes each, where index and FP64
-// position were a gather of 36; the FP64 positions are fetched only for a pair
-// in the test's uncertain band.  Against a candidate-by-candidate walk, and
-// with the gather in between: 4,096 touching spheres 40.7 -> 11.5 -> 10.1 us
-// (eight lanes; one lane with its loads unrolled took 24.5), 64,000
-// 36.0 -> 26.1 -> 25.2 us, 10^6 falling spheres 108 -> 94 -> 84 us (eight lanes
-// there: 343), a beam of 110,000 42 -> 32 us.
+// cell-ordered FP32 records; a ball's own record is fetched only for a pair in
+// the test's uncertain band (RECORD_FIGURES).  Against a candidate-by-candidate walk: 4,096
+// touching spheres 40.7 -> 11.5 us (eight lanes; one lane with its loads
+// unrolled took 24.5), 64,000 36.0 -> 26.1 us, 10^6 falling spheres 108 -> 94 us
+// (eight lanes there: 343).
 template <int kLanes>
 __global__ void __launch_bounds__(128, kLanes == 1 ? 6 : 8) k_dem_build_pairs(DemDev d) {
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
@@ -587,31 +591,47 @@ __global__ void __launch_bounds__(kBoxThreads) k_dem_wall_box(DemDev d) {
 // with candidates (with periodic ghosts: added to the ghost sums there).
 // (Not part of the finish: the candidate arrays and the law would set the
 // register budget of every ball's.)
-// Whether ball (ri, r) reaches triangle tj's axis-aligned box.
-__device__ __forceinline__ bool near_triangle(const DemDev& d, int tj, double3 ri, double r) {
+// One triangle of the table (place k of its order).
+struct TriRec {
+    double3 a, b, c;
+    int4 id;
+};
+__device__ __forceinline__ TriRec tri_rec(const DemDev& d, int k) {
+    return TriRec{xyz(d.trA[k]), xyz(d.trB[k]), xyz(d.trC[k]), d.trI[k]};
+}
+__global__ void k_dem_tri_records(DemDev d) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= d.nTri) return;
+    const int tj = d.triOrder[k];
     const int4 tv = d.tris[tj];
-    const double3 a = xyz(d.vglobal[tv.x]), bb = xyz(d.vglobal[tv.y]), c = xyz(d.vglobal[tv.z]);
-    const double cx = fmin(fmax(ri.x, fmin(a.x, fmin(bb.x, c.x))), fmax(a.x, fmax(bb.x, c.x)));
-    const double cy = fmin(fmax(ri.y, fmin(a.y, fmin(bb.y, c.y))), fmax(a.y, fmax(bb.y, c.y)));
-    const double cz = fmin(fmax(ri.z, fmin(a.z, fmin(bb.z, c.z))), fmax(a.z, fmax(bb.z, c.z)));
+    d.trA[k] = d.vglobal[tv.x];
+    d.trB[k] = d.vglobal[tv.y];
+    d.trC[k] = d.vglobal[tv.z];
+    d.trI[k] = make_int4(d.triKey[tj], tj, tv.w, d.wmat[tv.w]);
+}
+// Whether ball (ri, r) reaches the triangle's axis-aligned box.
+__device__ __forceinline__ bool near_triangle(const TriRec& t, double3 ri, double r) {
+    const double cx = fmin(fmax(ri.x, fmin(t.a.x, fmin(t.b.x, t.c.x))), fmax(t.a.x, fmax(t.b.x, t.c.x)));
+    const double cy = fmin(fmax(ri.y, fmin(t.a.y, fmin(t.b.y, t.c.y))), fmax(t.a.y, fmax(t.b.y, t.c.y)));
+    const double cz = fmin(fmax(ri.z, fmin(t.a.z, fmin(t.b.z, t.c.z))), fmax(t.a.z, fmax(t.b.z, t.c.z)));
     const double dx = ri.x - cx, dy = ri.y - cy, dz = ri.z - cz;
     return dx * dx + dy * dy + dz * dz <= r * r;
 }
 constexpr int kMaxTriPerBall = 32;
-constexpr int kFewTris = 4;     // candidates a ball's own thread handles
+constexpr int kFewTris = 2;     // candidates a ball's own lanes handle
 constexpr int kSmallMesh = 16;  // triangles up to which a ball looks through all of them
 // The contacts of ball i with its candidates tri[0..cnt): the springs' carry,
 // classification, de-duplication, the law and the row's stores.
-template <class R, int kRoom>
+template <class R>
 __device__ __forceinline__ void wall_contacts(const DemDev& d, int i, const double4& p4, const int* tri, int cnt,
                                               double dtWall) {
     const double3 ri = xyz(p4);
     double3 F = mk3(0, 0, 0), T = mk3(0, 0, 0);
     bool any = false;
     // springs: carry from this ball's previous candidate row
-    double3 sS[kRoom], sR[kRoom], sT[kRoom];
-    double3 cp[kRoom];
-    int type[kRoom];
+    double3 sS[kMaxTriPerBall], sR[kMaxTriPerBall], sT[kMaxTriPerBall];
+    double3 cp[kMaxTriPerBall];
+    int type[kMaxTriPerBall];
     const int oc = d.wcntOld ? d.wcntOld[i] : 0;
     for (int c = 0; c < cnt; c++) {
         sS[c] = sR[c] = sT[c] = mk3(0, 0, 0);
@@ -703,64 +723,194 @@ __device__ __forceinline__ void wall_contacts(const DemDev& d, int i, const doub
         d.torqueA[i] = d4(T, 0);
     }
 }
-// f(tj) for ball i's candidate triangles in the reference's stencil order.  A
-// small mesh's triangles are few enough to be looked through in that order (the
-// table's), each against the stencil by its cell: shorter than the stencil's
+// The same for at most kFewTris = 2 candidates on a pair of lanes (mask gm), lane
+// q taking candidate q: the usual ball at a wall (a plane of two triangles),
+// whose chain of loads and FP64 arithmetic is what a small scene's evaluation
+// waits for.  One candidate's code is half as long to fetch as two side by side.
+struct WallSprings {
+    double3 s, r, t;
+};
+__device__ __forceinline__ WallSprings wall_springs(const DemDev& d, const double4* S, const double4* Rr, const double4* Tt,
+                                                    size_t at) {
+    WallSprings w;
+    w.s = xyz(S[at]);
+    w.r = d.roll ? xyz(Rr[at]) : mk3(0, 0, 0);
+    w.t = d.tors ? xyz(Tt[at]) : mk3(0, 0, 0);
+    return w;
+}
+__device__ __forceinline__ double3 from_other(double3 v, unsigned gm) {
+    return mk3(__shfl_xor_sync(gm, v.x, 1), __shfl_xor_sync(gm, v.y, 1), __shfl_xor_sync(gm, v.z, 1));
+}
+template <class R>
+__device__ __forceinline__ void wall_contacts_two(const DemDev& d, int i, int q, unsigned gm, const double4& p4, int mine,
+                                                  int others, int cnt, double dtWall) {
+    const double3 ri = xyz(p4);
+    const double4 v4 = d.vel[i];
+    const double3 wi = xyz(d.angv[i]);
+    const int mi = d.mat[i];
+    const bool has = q < cnt;
+    const TriRec t = tri_rec(d, mine);
+    // the springs of this triangle's entry in the previous row
+    const double3 zero = mk3(0, 0, 0);
+    WallSprings w{zero, zero, zero};
+    const int oc = d.wcntOld && has ? d.wcntOld[i] : 0;
+    for (int e = 0; e < oc; e++) {
+        const size_t os = (size_t)e * d.N + i;
+        if (d.wtjOld[os] == t.id.y) {
+            w = wall_springs(d, d.wSOld, d.wROld, d.wTOld, os);
+            break;
+        }
+    }
+    double3 cp = zero;
+    const int type = has ? classify_sphere_triangle(ri, p4.w, t.a, t.b, t.c, cp) : kCtNone;
+    bool cancel = type == kCtNone;
+    if (cancel) w = WallSprings{zero, zero, zero};
+    if (cnt > 1) {
+        // a contact that is the other triangle's as well is dropped, its springs
+        // the other's (never both: the first rule that holds for one excludes it
+        // for the other)
+        const int otype = __shfl_xor_sync(gm, type, 1);
+        const double3 ocp = from_other(cp, gm);
+        const WallSprings o{from_other(w.s, gm), from_other(w.r, gm), from_other(w.t, gm)};
+        if (type != kCtNone && type != kCtFace && otype != kCtNone) {
+            bool copy = false;
+            if (otype == kCtFace) {
+                const TriRec u = tri_rec(d, others);
+                copy = len2(cross(cp - u.a, u.b - u.a)) < 1.e-20 || len2(cross(cp - u.b, u.c - u.b)) < 1.e-20 ||
+                       len2(cross(cp - u.a, u.c - u.a)) < 1.e-20;
+            } else if (otype == kCtEdge) {
+                copy = (type != kCtEdge || q == 1) && len2(cp - ocp) < 1.e-20;
+            } else {
+                copy = type == otype && q == 1 && len2(cp - ocp) < 1.e-20;
+            }
+            if (copy) {
+                w = o;
+                cancel = true;
+            }
+        }
+    }
+    double3 F = zero, T = zero;
+    const bool acts = !cancel && !(v4.w < 1.e-20);
+    if (acts) {
+        const int wj = t.id.z;
+        const double3 n = normalize(ri - cp);
+        const double delta = p4.w - len(ri - cp);
+        const double3 rj = xyz(d.wpos[wj]), vj = xyz(d.wvel[wj]), wwj = xyz(d.wangv[wj]);
+        const double3 vc = xyz(v4) + cross(wi, cp - ri) - (vj + cross(wwj, cp - rj));
+        const MatPair& mp = d.mats[pair_param_index(mi, t.id.w, d.nMat, d.cap)];
+        V<R> Fc, Tc;
+        contact_law<R>(mp, Fc, Tc, w.s, w.r, w.t, vc, wi - wwj, n, delta, 1. / v4.w, p4.w, dtWall, d.roll, d.tors);
+        F = up(Fc);
+        T = up(Tc) + cross(cp - ri, F);
+    }
+    if (has) {
+        const size_t at = (size_t)q * d.N + i;
+        d.wtj[at] = t.id.y;
+        d.wS[at] = d4(w.s, 0);
+        if (d.roll) d.wR[at] = d4(w.r, 0);
+        if (d.tors) d.wT[at] = d4(w.t, 0);
+    }
+    bool any = acts;
+    if (cnt > 1) {
+        F += from_other(F, gm);
+        T += from_other(T, gm);
+        any = __shfl_xor_sync(gm, (int)acts, 1) || acts;
+    }
+    if (q) return;
+    d.wcnt[i] = cnt;
+    if (d.accA) {
+        if (any) {
+            d.forceA[i] = d4(xyz(d.forceA[i]) + F, 0);
+            d.torqueA[i] = d4(xyz(d.torqueA[i]) + T, 0);
+        }
+    } else if (cnt) {
+        d.forceA[i] = d4(F, 0);
+        d.torqueA[i] = d4(T, 0);
+    }
+}
+
+// f(k, triangle) for ball i's candidate triangles (place k of the table) in the
+// reference's stencil order, taking every step-th of a row's triangles from
+// `first` on.  A small mesh's triangles are few enough to be looked through in
+// that order, each against the stencil by its cell: shorter than the stencil's
 // nine rows of bounds.
 template <class F>
-__device__ __forceinline__ void for_near_triangles(const DemDev& d, const double4& p4, F&& f) {
+__device__ __forceinline__ void for_near_triangles(const DemDev& d, const double4& p4, int first, int step, F&& f) {
     const double3 ri = xyz(p4);
     const Stencil st = stencil_of(ri, d.tg);
     if (d.nTri <= kSmallMesh) {
-        for (int k = 0; k < d.nTri; k++) {
-            const int tj = d.triOrder[k];
-            const int key = d.triKey[tj];
-            const int cx = key % d.tg.nx, cy = (key / d.tg.nx) % d.tg.ny, cz = key / (d.tg.nx * d.tg.ny);
-            if (cx < st.c.x + st.s.x || cx > st.c.x + st.e.x || cy < st.c.y + st.s.y || cy > st.c.y + st.e.y ||
-                cz < st.c.z + st.s.z || cz > st.c.z + st.e.z)
-                continue;
-            if (near_triangle(d, tj, ri, p4.w)) f(tj);
+        const int own = key_of(st.c, d.tg);
+        for (int k = first; k < d.nTri; k += step) {
+            const TriRec t = tri_rec(d, k);
+            const int rel = t.id.x - own;
+            bool in = false;  // the triangle's cell lies in a row of the stencil
+#pragma unroll
+            for (int r = 0; r < 9; r++) {
+                const int zz = r / 3 - 1, yy = r % 3 - 1;
+                const int x = rel - (zz * d.tg.ny + yy) * d.tg.nx;
+                in |= (zz >= st.s.z) & (zz <= st.e.z) & (yy >= st.s.y) & (yy <= st.e.y) & (x >= st.s.x) & (x <= st.e.x);
+            }
+            if (near_triangle(t, ri, p4.w) & in) f(k, t.id.y);
         }
         return;
     }
     for_stencil_rows(st, d.tg, d.triCellStart, [&](int b, int e) {
-        for (int k = b; k < e; k++) {
-            const int tj = d.triOrder[k];
-            if (near_triangle(d, tj, ri, p4.w)) f(tj);
+        for (int k = b + first; k < e; k += step) {
+            const TriRec t = tri_rec(d, k);
+            if (near_triangle(t, ri, p4.w)) f(k, t.id.y);
         }
     });
 }
-// A ball's wall contacts in its own thread, up to kFewTris candidates; a ball
+// Whether a ball lies within its radius (with a relative margin that covers
+// rounding) of the box of all mesh vertices: outside it no triangle passes the
+// candidate test.
+__device__ __forceinline__ bool near_mesh(const DemDev& d, double3 ri, double r) {
+    const double3 lo = xyz(d.wbox[0]), hi = xyz(d.wbox[1]);
+    const double dx = ri.x - fmin(fmax(ri.x, lo.x), hi.x), dy = ri.y - fmin(fmax(ri.y, lo.y), hi.y),
+                 dz = ri.z - fmin(fmax(ri.z, lo.z), hi.z);
+    return !(dx * dx + dy * dy + dz * dz > 1.000001 * r * r);
+}
+// A ball's wall contacts on a pair of lanes, up to kFewTris candidates; a ball
 // with more is listed for k_dem_walls_many, whose arrays of 32 would otherwise
-// set every ball's stack (10^6 falling spheres 20.0 -> 14.1 us; the large form
-// as a function called from here: 126 us, its frame is every thread's).
+// set every ball's stack.  4,096
+// bouncing spheres 29.7 -> 23.4 us a step against one thread per ball with up
+// to four candidates; 10^6 falling spheres 13.4 -> 11.3 us an evaluation.
 template <class R>
 __device__ __forceinline__ void walls_ball(const DemDev& d, int i, double dtWall) {
+    const int q = threadIdx.x & 1;
+    const unsigned gm = 3u << (threadIdx.x & 30);
     const double4 p4 = d.pos[i];
-    const double3 ri = xyz(p4);
-    {
-        // outside the mesh box by more than r (with a relative margin that
-        // covers rounding): no triangle passes the candidate test below
-        const double3 lo = xyz(d.wbox[0]), hi = xyz(d.wbox[1]);
-        const double cx = fmin(fmax(ri.x, lo.x), hi.x), cy = fmin(fmax(ri.y, lo.y), hi.y),
-                     cz = fmin(fmax(ri.z, lo.z), hi.z);
-        const double dx = ri.x - cx, dy = ri.y - cy, dz = ri.z - cz;
-        if (dx * dx + dy * dy + dz * dz > 1.000001 * p4.w * p4.w) {
-            d.wcnt[i] = 0;
-            return;
-        }
-    }
-    int tri[kFewTris];
-    int cnt = 0;
-    for_near_triangles(d, p4, [&](int tj) {
-        if (cnt < kFewTris) tri[cnt] = tj;
-        cnt++;
-    });
-    if (cnt > kFewTris) {
-        d.wmany[1 + atomicAdd(d.wmany, 1)] = i;
+    if (!near_mesh(d, xyz(p4), p4.w)) {
+        if (q == 0) d.wcnt[i] = 0;
         return;
     }
-    wall_contacts<R, kFewTris>(d, i, p4, tri, cnt, dtWall);
+    // each lane looks through every other triangle; the places of the table
+    // ascend along the stencil, so two hits are put in order by their places
+    int a = 0, b = 0, cnt = 0;
+    for_near_triangles(d, p4, q, 2, [&](int k, int) {
+        if (cnt == 0) a = k;
+        else if (cnt == 1) b = k;
+        cnt++;
+    });
+    __syncwarp(gm);
+    const int oa = __shfl_xor_sync(gm, a, 1), ob = __shfl_xor_sync(gm, b, 1), oc = __shfl_xor_sync(gm, cnt, 1);
+    if (cnt == 0) {
+        a = oa;
+        b = ob;
+    } else if (cnt == 1 && oc == 1) {
+        b = max(a, oa);
+        a = min(a, oa);
+    }
+    cnt += oc;
+    if (cnt > kFewTris) {
+        if (q == 0) d.wmany[1 + atomicAdd(d.wmany, 1)] = i;
+        return;
+    }
+    if (cnt == 0) {
+        if (q == 0) d.wcnt[i] = 0;
+    } else {
+        wall_contacts_two<R>(d, i, q, gm, p4, q ? b : a, q ? a : b, cnt, dtWall);
+    }
 }
 // The balls with more than kFewTris candidate triangles (wmany: their count,
 // then their indices; the finish of the evaluation clears the count).
@@ -773,7 +923,7 @@ __global__ void __launch_bounds__(128) k_dem_walls_many(DemDev d, double dtWall)
         const double4 p4 = d.pos[i];
         int tri[kMaxTriPerBall];
         int cnt = 0;
-        for_near_triangles(d, p4, [&](int tj) {
+        for_near_triangles(d, p4, 0, 1, [&](int, int tj) {
             if (cnt < d.KT && cnt < kMaxTriPerBall) tri[cnt] = tj;
             cnt++;
         });
@@ -782,14 +932,37 @@ __global__ void __launch_bounds__(128) k_dem_walls_many(DemDev d, double dtWall)
             atomicExch(&d.status->overflow, 1);
             cnt = min(d.KT, kMaxTriPerBall);
         }
-        wall_contacts<R, kMaxTriPerBall>(d, i, p4, tri, cnt, dtWall);
+        wall_contacts<R>(d, i, p4, tri, cnt, dtWall);
     }
 }
-template <class R>
-__global__ void __launch_bounds__(128) k_dem_walls(DemDev d, double dtWall) {
+// All balls, a pair of lanes each.  kSparse, for large scenes, most of whose
+// balls are far from the mesh: a warp looks at 32 balls, a lane each, and then
+// only those near the mesh get their pair.
+template <class R, bool kSparse>
+__device__ __forceinline__ void walls_part(const DemDev& d, int block, double dtWall) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (!kSparse) {
+        const int i = (block * blockDim.x + threadIdx.x) >> 1;
+        if (i < d.N) walls_ball<R>(d, i, dtWall);
+    } else {
+        __shared__ unsigned char place[4][32];  // the near lanes of each warp's 32 balls
+        const int w = threadIdx.x >> 5, i = block * blockDim.x + threadIdx.x;
+        bool near = false;
+        if (i < d.N) {
+            const double4 p4 = d.pos[i];
+            near = near_mesh(d, xyz(p4), p4.w);
+            if (!near) d.wcnt[i] = 0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, near);
+        if (near) place[w][__popc(m & ((1u << lane) - 1u))] = (unsigned char)lane;
+        __syncwarp();
+        for (int k = lane >> 1; k < __popc(m); k += 16) walls_ball<R>(d, i - lane + place[w][k], dtWall);
+    }
+}
+template <class R, bool kSparse>
+__global__ void __launch_bounds__(128, 4) k_dem_walls(DemDev d, double dtWall) {
     chain_enter();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < d.N) walls_ball<R>(d, i, dtWall);
+    walls_part<R, kSparse>(d, blockIdx.x, dtWall);
 }
 // Small scenes, whose steps are bound by the latency of each launch's chain
 // of loads: the pairs, the bonds and the wall contacts, which do not depend on
@@ -809,10 +982,7 @@ __global__ void __launch_bounds__(128, 4) k_dem_forces(DemDev d, double dt, doub
         if (k < d.nBond) bond_force(d, k, dt, store);
         return;
     }
-    if constexpr (kWalls) {
-        const int i = (b - bondBlocks) * blockDim.x + threadIdx.x;
-        if (i < d.N) walls_ball<R>(d, i, dtWall);
-    }
+    if constexpr (kWalls) walls_part<R, false>(d, b - bondBlocks, dtWall);
 }
 
 // Per-ball finish of one force evaluation:
@@ -1331,7 +1501,8 @@ struct DemScene {
     DBuf<int> bpair;
     bool bondPairsStale = true;  // bpair does not describe the current pair list
     DBuf<double4> wpos, wvel, wangv, wq, vlocal, vglobal, tcenter;
-    DBuf<double4> wbox;
+    DBuf<double4> wbox, trA, trB, trC;
+    DBuf<int4> trI;
     DBuf<int> wmany;
     DBuf<int> wmat, vwall;
     DBuf<int4> tris;
@@ -1409,10 +1580,9 @@ struct DemScene {
         d.bincStart = bincStart.p; d.binc = binc.p;
         d.wpos = wpos.p; d.wvel = wvel.p; d.wangv = wangv.p; d.wq = wq.p; d.wmat = wmat.p;
         d.vlocal = vlocal.p; d.vglobal = vglobal.p; d.vwall = vwall.p; d.tris = tris.p; d.tcenter = tcenter.p;
-        d.rec = ballCells.rec.p;
-        d.triOrder = triCells.sorted.p; d.triKey = triCells.key.p; d.wmany = wmany.p; d.triCellStart = triCells.start.p; d.wbox = wbox.p;
+        d.triOrder = triCells.sorted.p; d.triKey = triCells.key.p; d.trA = trA.p; d.trB = trB.p; d.trC = trC.p; d.trI = trI.p; d.wmany = wmany.p; d.triCellStart = triCells.start.p; d.wbox = wbox.p;
         int wo = wcur ^ 1;
-        d.wtj = wtj[wcur].p; d.wcnt = wcnt[wcur].p; d.wS = wS[wcur].p; d.wR = wR[wcur].p; d.wT = wT[wcur].p;
+        d.wtj = wtj[wcur].p; d.wcnt = wcnt[wcur].p; d.rec = ballCells.rec.p; d.wS = wS[wcur].p; d.wR = wR[wcur].p; d.wT = wT[wcur].p;
         if (haveWallRows) {
             d.wtjOld = wtj[wo].p; d.wcntOld = wcnt[wo].p; d.wSOld = wS[wo].p; d.wROld = wR[wo].p; d.wTOld = wT[wo].p;
         }
@@ -1748,9 +1918,15 @@ struct DemScene {
         if (hTris.empty()) return;
         triCells.build(tcenter.p, (int)hTris.size(), s);
         if (wbox.n < 2) wbox.alloc(2, s, false);
+        const size_t nt = hTris.size();
+        if (trI.n < nt) {
+            trA.alloc(nt, s, false); trB.alloc(nt, s, false); trC.alloc(nt, s, false);
+            trI.alloc(nt, s, false);
+        }
         DemDev d = dev(false);
         k_dem_wall_box<<<1, kBoxThreads, 0, s>>>(d);
-        launch_count(1 + triCells.launches);
+        k_dem_tri_records<<<grid_for(nt, 128), 128, 0, s>>>(d);
+        launch_count(2 + triCells.launches);
     }
     // calculateBallContactForceTorque(dt) [+ addTriangleContactForceTorque(dtWall)]
     // [+ external hook at extTime] [+ half-step integration]
@@ -1772,6 +1948,8 @@ struct DemScene {
         }
         DemDev d = dev(false);
         d.accA = ghostSums ? 1 : 0;
+        const bool sparse = n > kChainBalls;
+        const unsigned wallGrid = grid_for((size_t)n * (sparse ? 1 : 2), 128);
         if (!doWalls) d.nTri = 0;
         if (d.nBond && bondPairsStale) bond_pairs(d);
         const int clumps = hCpos.empty() ? 0 : (pebblesInRange ? 2 : 1);
@@ -1781,7 +1959,7 @@ struct DemScene {
         const unsigned pairGrid = std::min(grid_for((size_t)n * 4, 128), (unsigned)device_sms() * 16);
         const unsigned bondGrid = grid_for(d.nBond, 128);
         if (chain && !ghostSums) {
-            const unsigned grid = pairGrid + bondGrid + (doWalls ? grid_for(n, 128) : 0);
+            const unsigned grid = pairGrid + bondGrid + (doWalls ? wallGrid : 0);
             auto go = [&](auto kernel) {
                 launch_chained(kernel, grid, 128, s, chain, d, dt, dtWall, store, (int)pairGrid, (int)bondGrid);
             };
@@ -1804,8 +1982,9 @@ struct DemScene {
                 launch_count(1);
             }
             if (doWalls) {
-                if (fp64) launch_chained(k_dem_walls<double>, grid_for(n, 128), 128, s, chain, d, dtWall);
-                else launch_chained(k_dem_walls<float>, grid_for(n, 128), 128, s, chain, d, dtWall);
+                auto go = [&](auto kernel) { launch_chained(kernel, wallGrid, 128, s, chain, d, dtWall); };
+                if (sparse) fp64 ? go(k_dem_walls<double, true>) : go(k_dem_walls<float, true>);
+                else fp64 ? go(k_dem_walls<double, false>) : go(k_dem_walls<float, false>);
                 launch_count(1);
             }
         }
