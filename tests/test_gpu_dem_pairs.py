@@ -90,7 +90,7 @@ def test_pairs_at_the_cut_off(gpu, n):
     np.testing.assert_array_equal(np.sort(pair_keys(*ab)), pair_keys(inside, inside + m))
 
 
-@pytest.mark.parametrize("n", [250_000, 275_000])  # 250,047 and 274,625: either side of the finish's lane limit (sparse walls)
+@pytest.mark.parametrize("n", [30_000, 36_000, 70_000])  # 29,791 and 35,937: either side of the finish's lane limit; sparse walls
 def test_finish_forms_agree_with_the_oracle(gpu, n):
     sc = scenes.dem_drop_poly(n, seed=2)
     rng = np.random.default_rng(1)

@@ -964,10 +964,11 @@ __global__ void __launch_bounds__(128, 4) k_dem_walls(DemDev d, double dtWall) {
     chain_enter();
     walls_part<R, kSparse>(d, blockIdx.x, dtWall);
 }
-// Small scenes, whose steps are bound by the latency of each launch's chain
-// of loads: the pairs, the bonds and the wall contacts, which do not depend on
-// one another, in one launch, each with its own range of blocks.
-template <class R, bool kWalls>
+// The pairs, the bonds and the wall contacts, which do not depend on one
+// another, in one launch, each with its own range of blocks (force_eval says
+// when).
+enum { kNoWalls, kDenseWalls, kSparseWalls };
+template <class R, int kWalls>
 __global__ void __launch_bounds__(128, 4) k_dem_forces(DemDev d, double dt, double dtWall, int store, int pairBlocks,
                                                        int bondBlocks) {
     chain_enter();
@@ -982,7 +983,7 @@ __global__ void __launch_bounds__(128, 4) k_dem_forces(DemDev d, double dt, doub
         if (k < d.nBond) bond_force(d, k, dt, store);
         return;
     }
-    if constexpr (kWalls) walls_part<R, false>(d, b - bondBlocks, dtWall);
+    if constexpr (kWalls) walls_part<R, kWalls == kSparseWalls>(d, b - bondBlocks, dtWall);
 }
 
 // Per-ball finish of one force evaluation:
@@ -1119,35 +1120,57 @@ __global__ void __launch_bounds__(128, 8)
 // pebbles: also sets the clump's pebbles (k_dem_pebbles, and their drift), when
 // every pebble lies in its clump's range and no hook runs in between: two
 // launches fewer per evaluation.
+// Four lanes share a clump: each sums, and afterwards sets, every fourth pebble
+// (a clump's chain of pebble loads, twice, is what the pass waits for).
+// 20,000 three-sphere clumps 5.6 -> 3.6 us.
+constexpr int kClumpLanes = 4;
 __global__ void __launch_bounds__(128) k_dem_clumps(DemDev d, double hdt, int first, int pebbles) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = t / kClumpLanes, sub = t % kClumpLanes;
     if (c >= d.nClump) return;
-    int2 pe = d.cpeb[c];
+    const unsigned gm = ((1u << kClumpLanes) - 1u) << ((threadIdx.x & 31) & ~(kClumpLanes - 1));
+    const int2 pe = d.cpeb[c];
     double3 cp = xyz(d.cpos[c]);
+    double3 v = xyz(d.cvel[c]), w = xyz(d.cangv[c]);
+    const double im = d.cinvm[c];
+    const double4 q = d.cq[c], Ia = d.cinvIa[c], Ib = d.cinvIb[c];
     double3 Fc = mk3(0, 0, 0), Tc = mk3(0, 0, 0);
-    for (int i = pe.x; i < pe.y; i++) {
-        double3 Fi = xyz(d.force[i]);
+    for (int i = pe.x + sub; i < pe.y; i += kClumpLanes) {
+        const double3 Fi = xyz(d.force[i]);
         Fc += Fi;
         Tc += xyz(d.torque[i]) + cross(xyz(d.pos[i]) - cp, Fi);
     }
-    d.cforce[c] = d4(Fc, 0);
-    d.ctorque[c] = d4(Tc, 0);
-    double im = d.cinvm[c];
-    double3 v = xyz(d.cvel[c]), w = xyz(d.cangv[c]);
-    double4 q = d.cq[c];
+#pragma unroll
+    for (int o = 1; o < kClumpLanes; o <<= 1) {
+        Fc.x += __shfl_xor_sync(gm, Fc.x, o);
+        Fc.y += __shfl_xor_sync(gm, Fc.y, o);
+        Fc.z += __shfl_xor_sync(gm, Fc.z, o);
+        Tc.x += __shfl_xor_sync(gm, Tc.x, o);
+        Tc.y += __shfl_xor_sync(gm, Tc.y, o);
+        Tc.z += __shfl_xor_sync(gm, Tc.z, o);
+    }
+    // every lane holds the same sums and advances the same state; lane 0 stores it,
+    // after all have read it
+    __syncwarp(gm);
     if (im > 1.e-20) {
         v += (Fc * im + d.gravity) * hdt;
-        w += rot_inv_inertia_apply(q, d.cinvIa[c], d.cinvIb[c], Tc) * hdt;
-        d.cvel[c] = d4(v, 0);
-        d.cangv[c] = d4(w, 0);
+        w += rot_inv_inertia_apply(q, Ia, Ib, Tc) * hdt;
     }
-    if (first) {
-        cp += (2.0 * hdt) * v;
-        d.cpos[c] = d4(cp, 0);
-        d.cq[c] = quat_rotate(q, w, 2.0 * hdt);
+    if (first) cp += (2.0 * hdt) * v;
+    if (sub == 0) {
+        d.cforce[c] = d4(Fc, 0);
+        d.ctorque[c] = d4(Tc, 0);
+        if (im > 1.e-20) {
+            d.cvel[c] = d4(v, 0);
+            d.cangv[c] = d4(w, 0);
+        }
+        if (first) {
+            d.cpos[c] = d4(cp, 0);
+            d.cq[c] = quat_rotate(q, w, 2.0 * hdt);
+        }
     }
     if (!pebbles) return;
-    for (int i = pe.x; i < pe.y; i++) {
+    for (int i = pe.x + sub; i < pe.y; i += kClumpLanes) {
         const double4 p = d.pos[i];
         const double3 u = v + cross(w, xyz(p) - cp);
         d.angv[i] = d4(w, 0);
@@ -1525,7 +1548,9 @@ struct DemScene {
     // mixed, the touching pack 53.9 -> 52.5; the 220k beam was 0.8% slower.
     static constexpr int kChainBalls = 65536;
     static constexpr int kBuildLaneBalls = 16384;  // up to this size eight lanes build a ball's row
-    static constexpr int kLaneBalls = 1 << 18;  // up to this size four lanes finish a ball
+    // Up to this size four lanes finish a ball (a beam of 110,000: 22.5 us on
+    // four, 14.5 on one; a pack of 64,000 the same either way).
+    static constexpr int kLaneBalls = 32768;
 
     // Periodic boundaries (setPeriodicBoundary, DEMSolver.h:1944-1959): one
     // ghost set per active direction, passed in the reference's order X, Y,
@@ -1958,13 +1983,18 @@ struct DemScene {
         const int fin = (clumps == 1 || hook) ? 0 : integ;
         const unsigned pairGrid = std::min(grid_for((size_t)n * 4, 128), (unsigned)device_sms() * 16);
         const unsigned bondGrid = grid_for(d.nBond, 128);
-        if (chain && !ghostSums) {
+        // one launch for small scenes (latency) and for bonds (their blocks and the
+        // pairs' fill each other's tails: a beam of 110,000 41.6 -> 34.0 us an
+        // evaluation); a million falling spheres' pairs and walls take 15.7 us either
+        // way, and the pairs alone fit a fifth block per SM
+        if ((chain || d.nBond) && !ghostSums) {
             const unsigned grid = pairGrid + bondGrid + (doWalls ? wallGrid : 0);
             auto go = [&](auto kernel) {
                 launch_chained(kernel, grid, 128, s, chain, d, dt, dtWall, store, (int)pairGrid, (int)bondGrid);
             };
-            if (fp64) doWalls ? go(k_dem_forces<double, true>) : go(k_dem_forces<double, false>);
-            else doWalls ? go(k_dem_forces<float, true>) : go(k_dem_forces<float, false>);
+            auto pick = [&](auto none, auto dense, auto wide) { !doWalls ? go(none) : sparse ? go(wide) : go(dense); };
+            if (fp64) pick(k_dem_forces<double, kNoWalls>, k_dem_forces<double, kDenseWalls>, k_dem_forces<double, kSparseWalls>);
+            else pick(k_dem_forces<float, kNoWalls>, k_dem_forces<float, kDenseWalls>, k_dem_forces<float, kSparseWalls>);
             launch_count(1);
         } else {
             if (fp64) launch_chained(k_dem_pairs<double>, pairGrid, 128, s, chain, d, dt);
@@ -2013,7 +2043,7 @@ struct DemScene {
         if (hook) run_hook(extTime);
         if (integ && clumps) {
             const bool own = fin == 0;  // the pebbles and the free balls in passes of their own
-            k_dem_clumps<<<grid_for(d.nClump, 128), 128, 0, s>>>(d, hdt, integ == 1, own ? 0 : 1);
+            k_dem_clumps<<<grid_for((size_t)d.nClump * kClumpLanes, 128), 128, 0, s>>>(d, hdt, integ == 1, own ? 0 : 1);
             launch_count(1);
             if (own) {
                 k_dem_pebbles<<<grid_for(n, 256), 256, 0, s>>>(d);
