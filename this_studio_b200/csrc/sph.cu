@@ -1871,9 +1871,9 @@ __device__ __forceinline__ void skin_pairs(int cnt, const int* __restrict__ nbV,
     if (lig == 0) cntOut[i] = over ? -1 : (kLaneRows | lanes);
 }
 
-// Resident blocks.  The first pass spills in its loops beyond 8 (128,000:
-// 58 us at 8, 61 at 9, 73 at 10); the second fits 9 (a million: 296 us at 8, 280
-// at 9, 296 at 10).
+// Resident blocks.  First pass: 61 us at 7 blocks, 64 at 8 (128,000), 438 and
+// 431 (a million); 9 and 10 spill in its loops (5% and 26% longer than 8).  The
+// second fits 9 (a million: 296 us at 8, 280 at 9, 296 at 10).
 template <bool kSkin, bool kMarkers>
 constexpr int kUniAccelBlocks = kMarkers || kSkin ? 8 : 9;
 template <bool kSkin, bool kMarkers = false, int kLanes = kQuad>
