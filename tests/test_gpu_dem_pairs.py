@@ -141,3 +141,50 @@ def test_walls_of_few_and_many_triangles(gpu, segments):
     p, q = g.getPairs(1), o.pairs(1)
     np.testing.assert_array_equal(pair_keys(p["objectPointed"], p["objectPointing"]), pair_keys(q["a"], q["b"]))
     assert len(p["objectPointed"]) > 0
+
+
+def _boxed(n_side, faces=6, **kw):
+    """A touching pack pressed against the faces of its box (two triangles a
+    face, first the floor): a ball on an edge or in a corner has four or six
+    candidate triangles."""
+    sc = scenes.dem_pack(n_side=n_side, **kw)
+    r = sc.radius[0]
+    (x0, y0, z0), (x1, y1, z1) = sc.position.min(0) - 0.97 * r, sc.position.max(0) + 0.97 * r
+    v = np.array([[x, y, z] for z in (z0, z1) for x, y in ((x0, y0), (x1, y0), (x1, y1), (x0, y1))])
+    q = [(0, 1, 2, 3), (0, 1, 5, 4), (1, 2, 6, 5), (2, 3, 7, 6), (3, 0, 4, 7), (4, 5, 6, 7)][:faces]
+    t = np.array([(a, b, c) for a, b, c, _ in q] + [(a, c, d) for a, _, c, d in q], np.int32)
+    sc.walls = [dict(vertices=v, tri0=t[:, 0], tri1=t[:, 1], tri2=t[:, 2], position=(0.0, 0.0, 0.0), material=0)]
+    return sc
+
+
+@pytest.mark.parametrize("n_side", [2, 9, 41])  # every ball in a corner; a small scene; 68,921: the sparse form
+def test_balls_on_the_edges_and_in_the_corners_of_a_box(gpu, n_side):
+    """Wall pairs as the oracle's, and the springs they carry over the steps
+    (rolling and torsion among them); 1e-9 against the oracle as the pack's
+    contacts amplify the rounding of an evaluation."""
+    g, o = _compare(_boxed(n_side), (1, 9) if n_side < 40 else (2,), tol=1e-9)
+    p, q = g.getPairs(1), o.pairs(1)
+    np.testing.assert_array_equal(pair_keys(p["objectPointed"], p["objectPointing"]), pair_keys(q["a"], q["b"]))
+    assert np.bincount(p["objectPointed"]).max() > 2
+    for k in ("sliding", "rolling", "torsion"):
+        assert rel_err(p[k], q[k]) < 1e-8, k
+
+
+def test_corners_do_not_hold_up_a_step(gpu):
+    """The few balls with more than two candidate triangles are not what a step
+    waits for: a boxed pack takes 2.5 times the step of one on a floor alone
+    (its six faces' contacts included), and took 5.2 times when each such ball
+    searched and settled its contacts in one thread."""
+    import time
+
+    def step_us(sc):
+        s = build_dem(sc, "mixed")
+        best = 1e9
+        for _ in range(6):
+            t0 = time.perf_counter()
+            s.step(200)
+            s.getBall()
+            best = min(best, time.perf_counter() - t0)
+        return best
+
+    assert step_us(_boxed(16)) < 3.7 * step_us(_boxed(16, faces=1))

@@ -582,15 +582,6 @@ __global__ void __launch_bounds__(kBoxThreads) k_dem_wall_box(DemDev d) {
     }
 }
 
-// Mesh-wall contacts of one force evaluation, per ball: candidate triangles
-// by AABB over the triangle grid with spring carry
-// (count/writeBallTriangleInteractionsKernel, ballNeighborSearchKernel.cu:153-338),
-// edge/vertex de-duplication (updateBallTriangleContact, contactKernel.cu:261-418)
-// and the wall law (calBallWallContactForceTorqueKernel, contactKernel.cu:420-533),
-// written to the ball's accumulators, which k_dem_finalize reads for balls
-// with candidates (with periodic ghosts: added to the ghost sums there).
-// (Not part of the finish: the candidate arrays and the law would set the
-// register budget of every ball's.)
 // One triangle of the table (place k of its order).
 struct TriRec {
     double3 a, b, c;
@@ -620,113 +611,15 @@ __device__ __forceinline__ bool near_triangle(const TriRec& t, double3 ri, doubl
 constexpr int kMaxTriPerBall = 32;
 constexpr int kFewTris = 2;     // candidates a ball's own lanes handle
 constexpr int kSmallMesh = 16;  // triangles up to which a ball looks through all of them
-// The contacts of ball i with its candidates tri[0..cnt): the springs' carry,
-// classification, de-duplication, the law and the row's stores.
-template <class R>
-__device__ __forceinline__ void wall_contacts(const DemDev& d, int i, const double4& p4, const int* tri, int cnt,
-                                              double dtWall) {
-    const double3 ri = xyz(p4);
-    double3 F = mk3(0, 0, 0), T = mk3(0, 0, 0);
-    bool any = false;
-    // springs: carry from this ball's previous candidate row
-    double3 sS[kMaxTriPerBall], sR[kMaxTriPerBall], sT[kMaxTriPerBall];
-    double3 cp[kMaxTriPerBall];
-    int type[kMaxTriPerBall];
-    const int oc = d.wcntOld ? d.wcntOld[i] : 0;
-    for (int c = 0; c < cnt; c++) {
-        sS[c] = sR[c] = sT[c] = mk3(0, 0, 0);
-        for (int q = 0; q < oc; q++) {
-            size_t os = (size_t)q * d.N + i;
-            if (d.wtjOld[os] == tri[c]) {
-                sS[c] = xyz(d.wSOld[os]);
-                if (d.roll) sR[c] = xyz(d.wROld[os]);
-                if (d.tors) sT[c] = xyz(d.wTOld[os]);
-                break;
-            }
-        }
-        int4 tv = d.tris[tri[c]];
-        cp[c] = mk3(0, 0, 0);
-        type[c] = classify_sphere_triangle(ri, p4.w, xyz(d.vglobal[tv.x]), xyz(d.vglobal[tv.y]),
-                                           xyz(d.vglobal[tv.z]), cp[c]);
-    }
-    // de-duplication, sequential as in the reference thread
-    unsigned cancel = 0;
-    for (int c = 0; c < cnt; c++) {
-        if (type[c] == kCtNone) {
-            sS[c] = sR[c] = sT[c] = mk3(0, 0, 0);
-            cancel |= 1u << c;
-            continue;
-        }
-        if (type[c] == kCtFace) continue;
-        for (int c1 = 0; c1 < cnt; c1++) {
-            if (c1 == c) continue;
-            int t1 = type[c1];
-            bool copy = false;
-            if (t1 == kCtNone) continue;
-            if (t1 == kCtFace) {
-                int4 tv = d.tris[tri[c1]];
-                double3 q0 = xyz(d.vglobal[tv.x]), q1 = xyz(d.vglobal[tv.y]), q2 = xyz(d.vglobal[tv.z]);
-                if (len2(cross(cp[c] - q0, q1 - q0)) < 1.e-20) copy = true;
-                else if (len2(cross(cp[c] - q1, q2 - q1)) < 1.e-20) copy = true;
-                else if (len2(cross(cp[c] - q0, q2 - q0)) < 1.e-20) copy = true;
-            } else if (t1 == kCtEdge) {
-                if (type[c] == t1) { if (c1 < c && len2(cp[c] - cp[c1]) < 1.e-20) copy = true; }
-                else if (len2(cp[c] - cp[c1]) < 1.e-20) copy = true;
-            } else {
-                if (type[c] == t1 && c1 < c && len2(cp[c] - cp[c1]) < 1.e-20) copy = true;
-            }
-            if (copy) {
-                sS[c] = sS[c1]; sR[c] = sR[c1]; sT[c] = sT[c1];
-                cancel |= 1u << c;
-                break;
-            }
-        }
-    }
-    // wall law (fixed balls skip it, as calBallWallContactForceTorqueKernel returns early)
-    const double4 v4 = cnt ? d.vel[i] : make_double4(0, 0, 0, 0);
-    if (cnt && !(v4.w < 1.e-20)) {
-        const double3 vi = xyz(v4), wi = xyz(d.angv[i]);
-        const double m = 1. / v4.w;
-        const int mi = d.mat[i];
-        for (int c = 0; c < cnt; c++) {
-            if (cancel & (1u << c)) continue;
-            int wj = d.tris[tri[c]].w;
-            double3 n = normalize(ri - cp[c]);
-            double delta = p4.w - len(ri - cp[c]);
-            double3 rj = xyz(d.wpos[wj]), vj = xyz(d.wvel[wj]), wwj = xyz(d.wangv[wj]);
-            double3 vc = vi + cross(wi, cp[c] - ri) - (vj + cross(wwj, cp[c] - rj));
-            double3 wij = wi - wwj;
-            const MatPair mp = d.mats[pair_param_index(mi, d.wmat[wj], d.nMat, d.cap)];
-            V<R> Fc, Tc;
-            contact_law<R>(mp, Fc, Tc, sS[c], sR[c], sT[c], vc, wij, n, delta, m, p4.w, dtWall, d.roll, d.tors);
-            double3 Fd = up(Fc);
-            F += Fd;
-            T += up(Tc) + cross(cp[c] - ri, Fd);
-            any = true;
-        }
-    }
-    for (int c = 0; c < cnt; c++) {
-        size_t s = (size_t)c * d.N + i;
-        d.wtj[s] = tri[c];
-        d.wS[s] = d4(sS[c], 0);
-        if (d.roll) d.wR[s] = d4(sR[c], 0);
-        if (d.tors) d.wT[s] = d4(sT[c], 0);
-    }
-    d.wcnt[i] = cnt;
-    if (d.accA) {
-        if (any) {
-            d.forceA[i] = d4(xyz(d.forceA[i]) + F, 0);
-            d.torqueA[i] = d4(xyz(d.torqueA[i]) + T, 0);
-        }
-    } else if (cnt) {
-        d.forceA[i] = d4(F, 0);
-        d.torqueA[i] = d4(T, 0);
-    }
-}
-// The same for at most kFewTris = 2 candidates on a pair of lanes (mask gm), lane
-// q taking candidate q: the usual ball at a wall (a plane of two triangles),
-// whose chain of loads and FP64 arithmetic is what a small scene's evaluation
-// waits for.  One candidate's code is half as long to fetch as two side by side.
+// Mesh-wall contacts of one force evaluation, per ball: candidate triangles
+// by AABB over the triangle grid with spring carry
+// (count/writeBallTriangleInteractionsKernel, ballNeighborSearchKernel.cu:153-338),
+// edge/vertex de-duplication (updateBallTriangleContact, contactKernel.cu:261-418)
+// and the wall law (calBallWallContactForceTorqueKernel, contactKernel.cu:420-533),
+// written to the ball's accumulators, which k_dem_finalize reads for balls
+// with candidates (with periodic ghosts: added to the ghost sums there).
+// (Not part of the finish: the law would set the register budget of every
+// ball's.)
 struct WallSprings {
     double3 s, r, t;
 };
@@ -738,85 +631,45 @@ __device__ __forceinline__ WallSprings wall_springs(const DemDev& d, const doubl
     w.t = d.tors ? xyz(Tt[at]) : mk3(0, 0, 0);
     return w;
 }
-__device__ __forceinline__ double3 from_other(double3 v, unsigned gm) {
-    return mk3(__shfl_xor_sync(gm, v.x, 1), __shfl_xor_sync(gm, v.y, 1), __shfl_xor_sync(gm, v.z, 1));
-}
-template <class R>
-__device__ __forceinline__ void wall_contacts_two(const DemDev& d, int i, int q, unsigned gm, const double4& p4, int mine,
-                                                  int others, int cnt, double dtWall) {
-    const double3 ri = xyz(p4);
-    const double4 v4 = d.vel[i];
-    const double3 wi = xyz(d.angv[i]);
-    const int mi = d.mat[i];
-    const bool has = q < cnt;
-    const TriRec t = tri_rec(d, mine);
-    // the springs of this triangle's entry in the previous row
+// The springs of triangle tj's entry in ball i's previous row (zeros: it has none).
+__device__ __forceinline__ WallSprings carried_springs(const DemDev& d, int i, int tj, int oldCnt) {
     const double3 zero = mk3(0, 0, 0);
-    WallSprings w{zero, zero, zero};
-    const int oc = d.wcntOld && has ? d.wcntOld[i] : 0;
-    for (int e = 0; e < oc; e++) {
+    for (int e = 0; e < oldCnt; e++) {
         const size_t os = (size_t)e * d.N + i;
-        if (d.wtjOld[os] == t.id.y) {
-            w = wall_springs(d, d.wSOld, d.wROld, d.wTOld, os);
-            break;
-        }
+        if (d.wtjOld[os] == tj) return wall_springs(d, d.wSOld, d.wROld, d.wTOld, os);
     }
-    double3 cp = zero;
-    const int type = has ? classify_sphere_triangle(ri, p4.w, t.a, t.b, t.c, cp) : kCtNone;
-    bool cancel = type == kCtNone;
-    if (cancel) w = WallSprings{zero, zero, zero};
-    if (cnt > 1) {
-        // a contact that is the other triangle's as well is dropped, its springs
-        // the other's (never both: the first rule that holds for one excludes it
-        // for the other)
-        const int otype = __shfl_xor_sync(gm, type, 1);
-        const double3 ocp = from_other(cp, gm);
-        const WallSprings o{from_other(w.s, gm), from_other(w.r, gm), from_other(w.t, gm)};
-        if (type != kCtNone && type != kCtFace && otype != kCtNone) {
-            bool copy = false;
-            if (otype == kCtFace) {
-                const TriRec u = tri_rec(d, others);
-                copy = len2(cross(cp - u.a, u.b - u.a)) < 1.e-20 || len2(cross(cp - u.b, u.c - u.b)) < 1.e-20 ||
-                       len2(cross(cp - u.a, u.c - u.a)) < 1.e-20;
-            } else if (otype == kCtEdge) {
-                copy = (type != kCtEdge || q == 1) && len2(cp - ocp) < 1.e-20;
-            } else {
-                copy = type == otype && q == 1 && len2(cp - ocp) < 1.e-20;
-            }
-            if (copy) {
-                w = o;
-                cancel = true;
-            }
-        }
-    }
-    double3 F = zero, T = zero;
-    const bool acts = !cancel && !(v4.w < 1.e-20);
-    if (acts) {
-        const int wj = t.id.z;
-        const double3 n = normalize(ri - cp);
-        const double delta = p4.w - len(ri - cp);
-        const double3 rj = xyz(d.wpos[wj]), vj = xyz(d.wvel[wj]), wwj = xyz(d.wangv[wj]);
-        const double3 vc = xyz(v4) + cross(wi, cp - ri) - (vj + cross(wwj, cp - rj));
-        const MatPair& mp = d.mats[pair_param_index(mi, t.id.w, d.nMat, d.cap)];
-        V<R> Fc, Tc;
-        contact_law<R>(mp, Fc, Tc, w.s, w.r, w.t, vc, wi - wwj, n, delta, 1. / v4.w, p4.w, dtWall, d.roll, d.tors);
-        F = up(Fc);
-        T = up(Tc) + cross(cp - ri, F);
-    }
-    if (has) {
-        const size_t at = (size_t)q * d.N + i;
-        d.wtj[at] = t.id.y;
-        d.wS[at] = d4(w.s, 0);
-        if (d.roll) d.wR[at] = d4(w.r, 0);
-        if (d.tors) d.wT[at] = d4(w.t, 0);
-    }
-    bool any = acts;
-    if (cnt > 1) {
-        F += from_other(F, gm);
-        T += from_other(T, gm);
-        any = __shfl_xor_sync(gm, (int)acts, 1) || acts;
-    }
-    if (q) return;
+    return WallSprings{zero, zero, zero};
+}
+// Whether the contact point cp, an edge's or a vertex', lies on an edge of triangle u.
+__device__ __forceinline__ bool on_an_edge(double3 cp, const TriRec& u) {
+    return len2(cross(cp - u.a, u.b - u.a)) < 1.e-20 || len2(cross(cp - u.b, u.c - u.b)) < 1.e-20 ||
+           len2(cross(cp - u.a, u.c - u.a)) < 1.e-20;
+}
+// The wall law of one contact: springs renewed, force and torque on the ball.
+template <class R>
+__device__ __forceinline__ void wall_law(const DemDev& d, const double4& p4, const double4& v4, double3 wi, int mi,
+                                         const TriRec& t, double3 cp, WallSprings& w, double dtWall, double3& F,
+                                         double3& T) {
+    const double3 ri = xyz(p4);
+    const int wj = t.id.z;
+    const double3 n = normalize(ri - cp);
+    const double delta = p4.w - len(ri - cp);
+    const double3 rj = xyz(d.wpos[wj]), vj = xyz(d.wvel[wj]), wwj = xyz(d.wangv[wj]);
+    const double3 vc = xyz(v4) + cross(wi, cp - ri) - (vj + cross(wwj, cp - rj));
+    const MatPair& mp = d.mats[pair_param_index(mi, t.id.w, d.nMat, d.cap)];
+    V<R> Fc, Tc;
+    contact_law<R>(mp, Fc, Tc, w.s, w.r, w.t, vc, wi - wwj, n, delta, 1. / v4.w, p4.w, dtWall, d.roll, d.tors);
+    F = up(Fc);
+    T = up(Tc) + cross(cp - ri, F);
+}
+__device__ __forceinline__ void store_wall_springs(const DemDev& d, size_t at, int tj, const WallSprings& w) {
+    d.wtj[at] = tj;
+    d.wS[at] = d4(w.s, 0);
+    if (d.roll) d.wR[at] = d4(w.r, 0);
+    if (d.tors) d.wT[at] = d4(w.t, 0);
+}
+// A ball's wall sums: `any` = some candidate acts.
+__device__ __forceinline__ void store_wall_sums(const DemDev& d, int i, int cnt, bool any, double3 F, double3 T) {
     d.wcnt[i] = cnt;
     if (d.accA) {
         if (any) {
@@ -828,8 +681,71 @@ __device__ __forceinline__ void wall_contacts_two(const DemDev& d, int i, int q,
         d.torqueA[i] = d4(T, 0);
     }
 }
+__device__ __forceinline__ double3 from_other(double3 v, unsigned gm) {
+    return mk3(__shfl_xor_sync(gm, v.x, 1), __shfl_xor_sync(gm, v.y, 1), __shfl_xor_sync(gm, v.z, 1));
+}
+// At most kFewTris = 2 candidates on a pair of lanes (mask gm), lane q taking
+// candidate q: the usual ball at a wall (a plane of two triangles), whose chain
+// of loads and FP64 arithmetic is what a small scene's evaluation waits for.
+// One candidate's code is half as long to fetch as two side by side.
+template <class R>
+__device__ __forceinline__ void wall_contacts_two(const DemDev& d, int i, int q, unsigned gm, const double4& p4, int mine,
+                                                  int others, int cnt, double dtWall) {
+    const double4 v4 = d.vel[i];
+    const double3 wi = xyz(d.angv[i]);
+    const int mi = d.mat[i];
+    const bool has = q < cnt;
+    const TriRec t = tri_rec(d, mine);
+    const double3 zero = mk3(0, 0, 0);
+    WallSprings w = carried_springs(d, i, t.id.y, d.wcntOld && has ? d.wcntOld[i] : 0);
+    double3 cp = zero;
+    const int type = has ? classify_sphere_triangle(xyz(p4), p4.w, t.a, t.b, t.c, cp) : kCtNone;
+    bool cancel = type == kCtNone;
+    if (cancel) w = WallSprings{zero, zero, zero};
+    if (cnt > 1) {
+        // a contact that is the other triangle's as well is dropped, its springs
+        // the other's (never both: the first rule that holds for one excludes it
+        // for the other)
+        const int otype = __shfl_xor_sync(gm, type, 1);
+        const double3 ocp = from_other(cp, gm);
+        const WallSprings o{from_other(w.s, gm), from_other(w.r, gm), from_other(w.t, gm)};
+        if (type != kCtNone && type != kCtFace && otype != kCtNone) {
+            bool copy = false;
+            if (otype == kCtFace) copy = on_an_edge(cp, tri_rec(d, others));
+            else if (otype == kCtEdge) copy = (type != kCtEdge || q == 1) && len2(cp - ocp) < 1.e-20;
+            else copy = type == otype && q == 1 && len2(cp - ocp) < 1.e-20;
+            if (copy) {
+                w = o;
+                cancel = true;
+            }
+        }
+    }
+    double3 F = zero, T = zero;
+    const bool acts = !cancel && !(v4.w < 1.e-20);
+    if (acts) wall_law<R>(d, p4, v4, wi, mi, t, cp, w, dtWall, F, T);
+    if (has) store_wall_springs(d, (size_t)q * d.N + i, t.id.y, w);
+    bool any = acts;
+    if (cnt > 1) {
+        F += from_other(F, gm);
+        T += from_other(T, gm);
+        any = __shfl_xor_sync(gm, (int)acts, 1) || acts;
+    }
+    if (q == 0) store_wall_sums(d, i, cnt, any, F, T);
+}
 
-// f(k, triangle) for ball i's candidate triangles (place k of the table) in the
+// Whether a triangle's cell lies in a row of the stencil.
+__device__ __forceinline__ bool in_stencil(const DemDev& d, const Stencil& st, int key) {
+    const int rel = key - key_of(st.c, d.tg);
+    bool in = false;
+#pragma unroll
+    for (int r = 0; r < 9; r++) {
+        const int zz = r / 3 - 1, yy = r % 3 - 1;
+        const int x = rel - (zz * d.tg.ny + yy) * d.tg.nx;
+        in |= (zz >= st.s.z) & (zz <= st.e.z) & (yy >= st.s.y) & (yy <= st.e.y) & (x >= st.s.x) & (x <= st.e.x);
+    }
+    return in;
+}
+// f(k) for the ball's candidate triangles (place k of the table) in the
 // reference's stencil order, taking every step-th of a row's triangles from
 // `first` on.  A small mesh's triangles are few enough to be looked through in
 // that order, each against the stencil by its cell: shorter than the stencil's
@@ -839,25 +755,16 @@ __device__ __forceinline__ void for_near_triangles(const DemDev& d, const double
     const double3 ri = xyz(p4);
     const Stencil st = stencil_of(ri, d.tg);
     if (d.nTri <= kSmallMesh) {
-        const int own = key_of(st.c, d.tg);
         for (int k = first; k < d.nTri; k += step) {
             const TriRec t = tri_rec(d, k);
-            const int rel = t.id.x - own;
-            bool in = false;  // the triangle's cell lies in a row of the stencil
-#pragma unroll
-            for (int r = 0; r < 9; r++) {
-                const int zz = r / 3 - 1, yy = r % 3 - 1;
-                const int x = rel - (zz * d.tg.ny + yy) * d.tg.nx;
-                in |= (zz >= st.s.z) & (zz <= st.e.z) & (yy >= st.s.y) & (yy <= st.e.y) & (x >= st.s.x) & (x <= st.e.x);
-            }
-            if (near_triangle(t, ri, p4.w) & in) f(k, t.id.y);
+            if (near_triangle(t, ri, p4.w) & in_stencil(d, st, t.id.x)) f(k);
         }
         return;
     }
     for_stencil_rows(st, d.tg, d.triCellStart, [&](int b, int e) {
         for (int k = b + first; k < e; k += step) {
             const TriRec t = tri_rec(d, k);
-            if (near_triangle(t, ri, p4.w)) f(k, t.id.y);
+            if (near_triangle(t, ri, p4.w)) f(k);
         }
     });
 }
@@ -871,8 +778,7 @@ __device__ __forceinline__ bool near_mesh(const DemDev& d, double3 ri, double r)
     return !(dx * dx + dy * dy + dz * dz > 1.000001 * r * r);
 }
 // A ball's wall contacts on a pair of lanes, up to kFewTris candidates; a ball
-// with more is listed for k_dem_walls_many, whose arrays of 32 would otherwise
-// set every ball's stack.  4,096
+// with more is listed for k_dem_walls_many.  4,096
 // bouncing spheres 29.7 -> 23.4 us a step against one thread per ball with up
 // to four candidates; 10^6 falling spheres 13.4 -> 11.3 us an evaluation.
 template <class R>
@@ -887,7 +793,7 @@ __device__ __forceinline__ void walls_ball(const DemDev& d, int i, double dtWall
     // each lane looks through every other triangle; the places of the table
     // ascend along the stencil, so two hits are put in order by their places
     int a = 0, b = 0, cnt = 0;
-    for_near_triangles(d, p4, q, 2, [&](int k, int) {
+    for_near_triangles(d, p4, q, 2, [&](int k) {
         if (cnt == 0) a = k;
         else if (cnt == 1) b = k;
         cnt++;
@@ -913,27 +819,113 @@ __device__ __forceinline__ void walls_ball(const DemDev& d, int i, double dtWall
     }
 }
 // The balls with more than kFewTris candidate triangles (wmany: their count,
-// then their indices; the finish of the evaluation clears the count).
+// then their indices; the finish of the evaluation clears the count), a warp
+// each: the lanes look through 32 triangles of a stencil row at a time, and lane
+// c takes candidate c.  (One thread per ball repeats the search and holds
+// arrays of 32 on its stack: 4,096 touching spheres in a box of twelve
+// triangles 108.7 -> 55.0 us a step, a sheet of 11,600 around a cylinder
+// of 2,664 triangles 871 -> 384.)
+struct WallShare {  // of a ball's candidates, among its warp
+    int place[kMaxTriPerBall];  // in the triangle table, ascending along the stencil
+    int type[kMaxTriPerBall];
+    int from[kMaxTriPerBall];  // the candidate whose contact (and springs) this one's is, or -1
+    double3 point[kMaxTriPerBall];
+};
+template <class R>
+__device__ __forceinline__ void wall_contacts_warp(const DemDev& d, int i, double dtWall, WallShare& sh) {
+    constexpr unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const double4 p4 = d.pos[i];
+    const double3 ri = xyz(p4);
+    const Stencil st = stencil_of(ri, d.tg);
+    int cnt = 0;
+    auto take = [&](bool near, int k) {
+        const unsigned m = __ballot_sync(all, near);
+        const int at = cnt + __popc(m & ((1u << lane) - 1u));
+        if (near && at < kMaxTriPerBall) sh.place[at] = k;
+        cnt += __popc(m);
+    };
+    __syncwarp();  // (the previous ball's entries are read)
+    if (d.nTri <= kSmallMesh) {
+        const bool here = lane < d.nTri;
+        const TriRec t = tri_rec(d, here ? lane : 0);
+        take(here && near_triangle(t, ri, p4.w) && in_stencil(d, st, t.id.x), lane);
+    } else {
+        for_stencil_rows(st, d.tg, d.triCellStart, [&](int b, int e) {
+            for (int k0 = b; k0 < e; k0 += 32) {
+                const int k = k0 + lane;
+                take(k < e && near_triangle(tri_rec(d, min(k, e - 1)), ri, p4.w), k);
+            }
+        });
+    }
+    if (cnt > d.KT || cnt > kMaxTriPerBall) {
+        if (lane == 0) {
+            atomicMax(&d.status->need_aux, cnt);
+            atomicExch(&d.status->overflow, 1);
+        }
+        cnt = min(d.KT, kMaxTriPerBall);
+    }
+    __syncwarp();
+    const bool has = lane < cnt;
+    const TriRec t = tri_rec(d, cnt ? sh.place[has ? lane : 0] : 0);
+    const double3 zero = mk3(0, 0, 0);
+    WallSprings w = carried_springs(d, i, t.id.y, d.wcntOld && has ? d.wcntOld[i] : 0);
+    double3 cp = zero;
+    const int type = has ? classify_sphere_triangle(ri, p4.w, t.a, t.b, t.c, cp) : kCtNone;
+    if (type == kCtNone) w = WallSprings{zero, zero, zero};
+    sh.type[lane] = type;
+    sh.point[lane] = cp;
+    __syncwarp();
+    // the first candidate, in order, that has the same contact
+    int from = -1;
+    if (type != kCtNone && type != kCtFace) {
+        for (int c = 0; c < cnt && from < 0; c++) {
+            const int o = sh.type[c];
+            if (c == lane || o == kCtNone) continue;
+            bool copy;
+            if (o == kCtFace) copy = on_an_edge(cp, tri_rec(d, sh.place[c]));
+            else copy = (o == type ? c < lane : o == kCtEdge) && len2(cp - sh.point[c]) < 1.e-20;
+            if (copy) from = c;
+        }
+    }
+    sh.from[lane] = from;
+    __syncwarp();
+    // its springs: the candidates are settled one after the other, so an earlier
+    // one hands on what it took itself, a later one its own
+    int root = lane;
+    for (int c = from; c >= 0; c = sh.from[c]) {
+        const bool later = c > root;
+        root = c;
+        if (later) break;
+    }
+    auto take3 = [&](double3 v) {
+        return mk3(__shfl_sync(all, v.x, root), __shfl_sync(all, v.y, root), __shfl_sync(all, v.z, root));
+    };
+    w.s = take3(w.s);
+    if (d.roll) w.r = take3(w.r);
+    if (d.tors) w.t = take3(w.t);
+    const double4 v4 = d.vel[i];
+    double3 F = zero, T = zero;
+    const bool acts = type != kCtNone && from < 0 && !(v4.w < 1.e-20);
+    if (acts) wall_law<R>(d, p4, v4, xyz(d.angv[i]), d.mat[i], t, cp, w, dtWall, F, T);
+    if (has) store_wall_springs(d, (size_t)lane * d.N + i, t.id.y, w);
+    // the sums in the candidates' order
+    const unsigned act = __ballot_sync(all, acts);
+    double3 Fs = zero, Ts = zero;
+    for (unsigned m = act; m; m &= m - 1) {
+        root = __ffs(m) - 1;
+        Fs += take3(F);
+        Ts += take3(T);
+    }
+    if (lane == 0) store_wall_sums(d, i, cnt, act != 0, Fs, Ts);
+}
 template <class R>
 __global__ void __launch_bounds__(128) k_dem_walls_many(DemDev d, double dtWall) {
     chain_enter();
+    __shared__ WallShare share[4];
+    const int w = threadIdx.x >> 5;
     const int n = d.wmany[0];
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const int i = d.wmany[1 + k];
-        const double4 p4 = d.pos[i];
-        int tri[kMaxTriPerBall];
-        int cnt = 0;
-        for_near_triangles(d, p4, 0, 1, [&](int, int tj) {
-            if (cnt < d.KT && cnt < kMaxTriPerBall) tri[cnt] = tj;
-            cnt++;
-        });
-        if (cnt > d.KT || cnt > kMaxTriPerBall) {
-            atomicMax(&d.status->need_aux, cnt);
-            atomicExch(&d.status->overflow, 1);
-            cnt = min(d.KT, kMaxTriPerBall);
-        }
-        wall_contacts<R>(d, i, p4, tri, cnt, dtWall);
-    }
+    for (int k = blockIdx.x * 4 + w; k < n; k += gridDim.x * 4) wall_contacts_warp<R>(d, d.wmany[1 + k], dtWall, share[w]);
 }
 // All balls, a pair of lanes each.  kSparse, for large scenes, most of whose
 // balls are far from the mesh: a warp looks at 32 balls, a lane each, and then
@@ -2019,7 +2011,7 @@ struct DemScene {
             }
         }
         if (doWalls && d.nTri > kFewTris) {
-            const unsigned grid = std::min(grid_for(n, 128), (unsigned)device_sms() * 4);
+            const unsigned grid = std::min(grid_for((size_t)n * 4, 128), (unsigned)device_sms() * 8);
             if (fp64) launch_chained(k_dem_walls_many<double>, grid, 128, s, chain, d, dtWall);
             else launch_chained(k_dem_walls_many<float>, grid, 128, s, chain, d, dtWall);
             launch_count(1);
