@@ -112,3 +112,40 @@ def test_pair_sets_with_particles_outside_the_domain(gpu, prec, width):
     for s in (g, ref):
         s.step(5)
     _same(g.getSPH(), ref.getSPH(), TOL[prec])
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [1, 4200])  # couples: sixteen lanes a particle; 8,400 particles: four
+@pytest.mark.parametrize("bad", ["velocity", "pressure", "far"])
+def test_a_blown_up_particle_reaches_as_far_as_the_kernel(gpu, prec, n, bad):
+    """Couples of particles 2% beyond the cutoff of each other, within the skin
+    of the lists.  One of each couple has an infinite velocity, a NaN pressure
+    or (as the step before such a one leaves it) a velocity that takes it out of
+    all numbers: the other falls freely, to the bit."""
+    dx = 0.01
+    rng = np.random.default_rng(2)
+    at = np.stack(np.unravel_index(np.arange(n), (17, 17, 17)), 1) * 0.1 + 0.1
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    pos = np.concatenate([at, at + 1.02 * 2.6 * dx * u])
+    s = WCSPHSolver()
+    s.addSPHs(pos, None, 10.0, dx, 1000.0, 1e-3)
+    s.initialize((0.0,) * 3, (1.9,) * 3, (0.0, 0.0, -9.81), 1e-5, prec)
+    vel, p = np.zeros_like(pos), np.zeros(2 * n)
+    if bad == "velocity":
+        vel[n:] = [np.inf, -np.inf, np.nan]
+    elif bad == "pressure":
+        p[n:] = np.nan
+    else:
+        vel[n:] = 1e300
+    s.setSPH(velocity=vel, pressure=p)
+    s.step(1)
+    got = s.getSPH()
+    assert len(s.getPairs(0)[0]) == 0
+    free = WCSPHSolver()
+    free.addSPHs(pos[:n], None, 10.0, dx, 1000.0, 1e-3)
+    free.initialize((0.0,) * 3, (1.9,) * 3, (0.0, 0.0, -9.81), 1e-5, prec)
+    free.step(1)
+    want = free.getSPH()
+    for k in ("position", "velocity", "acceleration", "density"):
+        np.testing.assert_array_equal(got[k][:n], want[k])

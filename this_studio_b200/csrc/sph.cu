@@ -1707,6 +1707,13 @@ __device__ __forceinline__ Acc2 acc2_scaled(const Acc2& a, double r) {
     const double3 t = r * acc2_sum(a);
     return Acc2{make_float2((float)t.x, 0.f), make_float2((float)t.y, 0.f), make_float2((float)t.z, 0.f)};
 }
+// t's first halves where ka, its second halves where kb, else a's.  A pair beyond
+// the cutoff is left out so: a zero weight would pass on an infinite or NaN
+// velocity or pressure one skin width farther than the kernel reaches.
+__device__ __forceinline__ Acc2 acc2_where(bool ka, bool kb, const Acc2& t, const Acc2& a) {
+    return Acc2{make_float2(ka ? t.x.x : a.x.x, kb ? t.x.y : a.x.y), make_float2(ka ? t.y.x : a.y.x, kb ? t.y.y : a.y.y),
+                make_float2(ka ? t.z.x : a.z.x, kb ? t.z.y : a.z.y)};
+}
 // v_j - v_i of two neighbours.
 __device__ __forceinline__ void rel_vel(const OwnU& o, const float4& a, const float4& b, float2& x, float2& y, float2& z) {
     x = make_float2(a.x - o.v.x, b.x - o.v.x);
@@ -1895,8 +1902,9 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
                        PairGeom p = pair_geom(o.q, qa, qb, u);
                        ka = cutoff_u(p.r2.x, u, d.pos, d.pos, i, a);
                        kb = two && cutoff_u(p.r2.y, u, d.pos, d.pos, i, b);
-                       p.f = make_float2(ka ? p.f.x : 0.f, kb ? p.f.y : 0.f);
-                       acc_fluid_u(o, p, va, vb, __int_as_float(qa.w), __int_as_float(qb.w), u, acc2);
+                       Acc2 t = acc2;
+                       acc_fluid_u(o, p, va, vb, __int_as_float(qa.w), __int_as_float(qb.w), u, t);
+                       acc2 = acc2_where(ka, kb, t, acc2);
                    });
         acc2 = acc2_scaled(acc2, u.aR);
         if (d.ND > 0) {
@@ -2119,8 +2127,8 @@ __global__ void __launch_bounds__(kSphBlock, kBlocks) k_sph_accel_u64(SphDev d, 
     const OwnD o = own_d(d, i);
     double3 acc = mk3(0, 0, 0);
     // two neighbours side by side, without a branch between them: their chains
-    // of FP64 operations overlap (a pair beyond the cutoff, or the missing second
-    // one, has its kernel factor zeroed)
+    // of FP64 operations overlap (the sums leave out a pair beyond the cutoff and
+    // the missing second one; acc2_where)
     auto fluid = [&](int a, int b, bool two, bool& ka, bool& kb) {
         const double4 xa = load32(d.xr + a), xb = load32(d.xr + b);
         const double4 va = load32(d.vp + a), vb = load32(d.vp + b);
@@ -2128,12 +2136,14 @@ __global__ void __launch_bounds__(kSphBlock, kBlocks) k_sph_accel_u64(SphDev d, 
         const double a2 = dot(ra, ra), b2 = dot(rb, rb);
         ka = !kSkin || (d.ud.cut2 - a2) >= 0.;
         kb = two && (!kSkin || (d.ud.cut2 - b2) >= 0.);
-        PairD p = pair_geom_d(ra, a2, d.ud), q = pair_geom_d(rb, b2, d.ud);
-        if (kSkin) p.f = ka ? p.f : 0.0;
-        q.f = kb ? q.f : 0.0;
+        const PairD p = pair_geom_d(ra, a2, d.ud), q = pair_geom_d(rb, b2, d.ud);
         const double3 da = xyz(va) - o.v, db = xyz(vb) - o.v;
-        add_momentum_d(o, p, dot(da, ra) * p.inv, va.w, xa.w, da, d.ud.pF, d.ud.bF, d.ud.cF, acc);
-        add_momentum_d(o, q, dot(db, rb) * q.inv, vb.w, xb.w, db, d.ud.pF, d.ud.bF, d.ud.cF, acc);
+        double3 t = acc;
+        add_momentum_d(o, p, dot(da, ra) * p.inv, va.w, xa.w, da, d.ud.pF, d.ud.bF, d.ud.cF, t);
+        t = mk3(ka ? t.x : acc.x, ka ? t.y : acc.y, ka ? t.z : acc.z);
+        acc = t;
+        add_momentum_d(o, q, dot(db, rb) * q.inv, vb.w, xb.w, db, d.ud.pF, d.ud.bF, d.ud.cF, t);
+        acc = mk3(kb ? t.x : acc.x, kb ? t.y : acc.y, kb ? t.z : acc.z);
     };
     auto dummy = [&](int j) {
         const double3 r = o.x - xyz(load32(d.dpos + j));
