@@ -1662,6 +1662,13 @@ __device__ __forceinline__ PairGeom pair_geom(const int4& q, const int4& a, cons
     p.r2 = __ffma2_rn(p.x, p.x, __ffma2_rn(p.y, p.y, __fmul2_rn(p.z, p.z)));
     p.inv = make_float2(rsqrt_approx(fmaxf(p.r2.x, 1e-30f)), rsqrt_approx(fmaxf(p.r2.y, 1e-30f)));
     p.r = __fmul2_rn(p.r2, p.inv);
+    // one Newton step for both: y + y (1 - x y^2) / 2.  (The approximation's error
+    // has one sign over all pairs, and t^3 takes it five times; without the step
+    // an acceleration is off by 7.3e-7 instead of 6.5e-7, a uniform divergence by
+    // -2.5e-8 instead of 3e-9.  A million: 945 us a step without, 938 with it.)
+    const float2 e = __fmul2_rn(two(0.5f), __ffma2_rn(make_float2(-p.r.x, -p.r.y), p.inv, two(1.0f)));
+    p.inv = __ffma2_rn(p.inv, e, p.inv);
+    p.r = __ffma2_rn(p.r, e, p.r);
     float2 t = __ffma2_rn(p.r, u.mh, two(1.0f));
     t = make_float2(fmaxf(t.x, 0.0f), fmaxf(t.y, 0.0f));
     p.f = __fmul2_rn(__fmul2_rn(__fmul2_rn(t, t), t), u.fC);
@@ -1699,13 +1706,6 @@ struct Acc2 {
 };
 __device__ __forceinline__ double3 acc2_sum(const Acc2& a) {
     return mk3((double)a.x.x + (double)a.x.y, (double)a.y.x + (double)a.y.y, (double)a.z.x + (double)a.z.y);
-}
-// The sum times r, as an accumulator again: between the fluid's and the dummies'
-// terms (in FP64 the fluid's sum would hold six registers through the dummy
-// loop: second pass at 128,000 40.1 us against 38.6).
-__device__ __forceinline__ Acc2 acc2_scaled(const Acc2& a, double r) {
-    const double3 t = r * acc2_sum(a);
-    return Acc2{make_float2((float)t.x, 0.f), make_float2((float)t.y, 0.f), make_float2((float)t.z, 0.f)};
 }
 // t's first halves where ka, its second halves where kb, else a's.  A pair beyond
 // the cutoff is left out so: a zero weight would pass on an infinite or NaN
@@ -1894,6 +1894,7 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
     const OwnU o = own_u(d, i);
     const float2 z2 = make_float2(0.f, 0.f);
     Acc2 acc2{z2, z2, z2};
+    double3 fluid;  // the fluid's sum, kept in FP64 through the dummies' loop
     if constexpr (kSkin) {
         skin_pairs<kLanes>(d.cntV[i], d.nbV, d.KF, i, d.nbF, d.cntF, d.pos, d.g, d.fStart, i,
                    [&](int a, int b, bool two, bool& ka, bool& kb) {
@@ -1906,7 +1907,8 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
                        acc_fluid_u(o, p, va, vb, __int_as_float(qa.w), __int_as_float(qb.w), u, t);
                        acc2 = acc2_where(ka, kb, t, acc2);
                    });
-        acc2 = acc2_scaled(acc2, u.aR);
+        fluid = u.aR * acc2_sum(acc2);
+        acc2 = Acc2{z2, z2, z2};
         if (d.ND > 0) {
             skin_pairs<kLanes>(d.cntVD[i], d.nbVD, d.KD, i, d.nbD, d.cntD, d.pos, d.g, d.dStart, -1,
                        [&](int a, int b, bool two, bool& ka, bool& kb) {
@@ -1925,7 +1927,8 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
             p.f.y = two ? p.f.y : 0.f;
             acc_fluid_u(o, p, va, vb, __int_as_float(qa.w), __int_as_float(qb.w), u, acc2);
         });
-        acc2 = acc2_scaled(acc2, u.aR);
+        fluid = u.aR * acc2_sum(acc2);
+        acc2 = Acc2{z2, z2, z2};
         if (d.ND > 0) {
             lane_pairs<kLanes>(d.cntD[i], d.nbD, d.KD, i, -1, d.pos, d.g, d.dStart, d.dpos, [&](int a, int b, bool two) {
                 PairGeom p = pair_geom(o.q, d.dposq[a], d.dposq[b], u);
@@ -1934,7 +1937,7 @@ __global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
             });
         }
     }
-    double3 a = u.aD * acc2_sum(acc2);
+    double3 a = u.aD * (fluid + acc2_sum(acc2));
     float3 acc = make_float3(0.f, 0.f, 0.f);
     if constexpr (kMarkers) {
         // as k_sph_accel: the fluid-marker skin row with the exact test the
