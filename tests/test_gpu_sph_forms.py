@@ -149,3 +149,56 @@ def test_a_blown_up_particle_reaches_as_far_as_the_kernel(gpu, prec, n, bad):
     want = free.getSPH()
     for k in ("position", "velocity", "acceleration", "density"):
         np.testing.assert_array_equal(got[k][:n], want[k])
+
+
+def _squeezed(n, seed=5):
+    """A tank whose lower half is pressed together to 0.55 of its height: up to
+    forty particles to a cell below, rows of 60 to 160 entries."""
+    sc = _scene(*n, seed=seed)
+    z = sc.fluid[:, 2]
+    mid = 0.5 * (z.min() + z.max())
+    sc.fluid[:, 2] = np.where(z < mid, mid - 0.55 * (mid - z), z)
+    sc.velocity *= 0.5
+    return sc
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [(28, 27, 25), (35, 34, 33)])  # 18,900 and 39,270
+def test_list_build_of_large_fluids(gpu, prec, n):
+    """A fluid large enough for the list build with a particle per lane, whose
+    cells hold more than a warp's 32 particles and more than a stage's 128
+    candidates: after every step the pairs are those of exact lists built from
+    the step's start, and the state stays with it (sums in another order)."""
+    sc = _squeezed(n)
+    a, b = _build(sc, prec, headroom=0.2), _build(sc, prec, skin=0.0, headroom=0.2)
+    a.setGraphs(False)  # (a replayed step leaves no lists to read after a change of state)
+    b.setGraphs(False)
+    assert a.skinStats()[0] > 0 and b.skinStats()[0] == 0
+    cell = np.floor((sc.fluid - np.array(sc.minb)) / (2.6 * sc.spacing * 1.04)).astype(int)
+    assert np.unique(cell, axis=0, return_counts=True)[1].max() > 32
+    for _ in range(6):
+        a.step(1)
+        b.step(1)
+        for w in (0, 1):
+            p, q = pair_keys(*a.getPairs(w)), pair_keys(*b.getPairs(w))
+            np.testing.assert_array_equal(np.sort(p), np.sort(q))
+        rows = np.bincount(a.getPairs(0)[0])
+        assert rows.max() > 128 and len(np.unique(rows % 8)) == 8
+        _same(a.getSPH(), b.getSPH(), TOL[prec])
+        x = b.getSPH()  # both go on from one state, so that no pair at the cutoff differs
+        a.setSPH(x["position"], x["velocity"], x["density"], x["pressure"], x["densityChange"])
+        b.setSPH(x["position"], x["velocity"], x["density"], x["pressure"], x["densityChange"])
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+def test_rows_of_a_large_fluid_overflow_and_are_walked(gpu, prec):
+    """As test_overflowed_rows_are_walked, at the size of the build with a
+    particle per lane."""
+    sc = _scene(35, 34, 33)
+    a, b = _build(sc, prec, headroom=0.0), _build(sc, prec, uniform=False, headroom=1.0)
+    pos = sc.fluid.copy()
+    pos[:, 2] *= 0.9
+    for s in (a, b):
+        s.setSPH(position=pos)
+        s.step(4)
+    _same(a.getSPH(), b.getSPH(), 1e-5)

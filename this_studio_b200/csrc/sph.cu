@@ -902,20 +902,22 @@ __device__ __forceinline__ void cell_skin_rows(int ps, int pe, const Stencil& st
 // layout: 4 entries of 8 consecutive objects).  Candidates are staged kRowStage
 // at a time, so a column never outgrows kRowStage entries.  Half the
 // instructions of the candidate-per-lane form above (ballots and scattered
-// stores); 128,000: 36.8 -> 31.0 us, a million 178 -> 150.
+// stores); 128,000: 36.8 -> 31.0 us, a million 178 -> 150.  (The pointers into
+// shared memory name the same bytes, written and read by turns: none of them
+// is restricted; the times are the same.)
 constexpr int kRowStage = 128;
 constexpr int kRowWords = kRowStage + kRowStage * 32 / 16;  // float4 of shared memory per warp: stage, columns
 __device__ __forceinline__ void cell_rows_by_lane(int ps, int pe, const Stencil& st, const GridDesc& g,
                                                   const int* __restrict__ cellStart, const float4* __restrict__ ownf,
                                                   const float4* __restrict__ otherf, float hi, bool same, int K,
                                                   int* __restrict__ nb, int* __restrict__ cnt, int* needMax,
-                                                  int* overflow, float4* __restrict__ shared) {
+                                                  int* overflow, float4* shared) {
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const float4* __restrict__ pairs = shared;  // (-x0, -x1, -y0, -y1), (-z0, -z1, j0, j1) of two candidates
-    float* __restrict__ stage = reinterpret_cast<float*>(shared);
-    unsigned char* __restrict__ column = reinterpret_cast<unsigned char*>(shared + kRowStage) + lane;
-    const unsigned char* __restrict__ columns = reinterpret_cast<unsigned char*>(shared + kRowStage);
+    const float4* pairs = shared;  // (-x0, -x1, -y0, -y1), (-z0, -z1, j0, j1) of two candidates
+    float* stage = reinterpret_cast<float*>(shared);
+    unsigned char* column = reinterpret_cast<unsigned char*>(shared + kRowStage) + lane;
+    const unsigned char* columns = reinterpret_cast<unsigned char*>(shared + kRowStage);
     // stencil row r: its first candidate and its place among all candidates
     int b = 0, len = 0;
     if (lane < 9) {
