@@ -40,3 +40,24 @@ def test_clump_and_bond_state_comes_back_whole(gpu):
     c = g.getClump()
     np.testing.assert_array_equal(c["position"], [k["centroid"] for k in sc.clumps])
     np.testing.assert_array_equal(c["orientation"], np.tile([1.0, 0, 0, 0], (40, 1)))
+
+
+def test_read_back_takes_no_device_memory(gpu):
+    """A scene that fills the device can still be read: the getters allocate
+    nothing there (the staging is host memory)."""
+    from .test_zz_no_alloc import _Pool
+
+    rng = np.random.default_rng(3)
+    n = 200_000
+    pos = np.stack(np.unravel_index(np.arange(n), (59, 59, 59)), 1) * 0.02 + rng.uniform(0, 0.005, (n, 3))
+    s = DEMSolver()
+    s.addBalls(pos, None, None, 0.005, 2500.0, 0)
+    s.initialize((-0.1,) * 3, (1.3,) * 3, (0, 0, -9.81), 1e-5)
+    g = build_dem(scenes.bonded_beam_clumps(nx=30, ny=5, nz=5, n_clumps=40), "fp64")
+    pool = _Pool()
+    pool.reset_high()
+    used = pool.attr(pool.USED)
+    np.testing.assert_array_equal(s.getBall()["position"], pos)
+    g.getBondedInteraction()
+    g.getClump()
+    assert pool.attr(pool.USED) == used and pool.attr(pool.USED_HIGH) == used

@@ -359,19 +359,21 @@ struct DBuf {
 
 static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
 
-// (x, y, z) of n records as packed doubles.
-static __global__ void k_take3(size_t n, const double4* __restrict__ src, double* __restrict__ dst) {
-    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const double4 a = src[t];
-    dst[3 * t] = a.x;
-    dst[3 * t + 1] = a.y;
-    dst[3 * t + 2] = a.z;
+// The doubles [first, first + count) of n records' packed (x, y, z), by a few
+// blocks (the link is what bounds it, and the SMs are another stream's too).
+static __global__ void k_take3(size_t first, size_t count, const double* __restrict__ src, double* __restrict__ dst) {
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x) {
+        const size_t w = first + t;
+        dst[t] = src[4 * (w / 3) + w % 3];
+    }
 }
-// A getter's device records into the caller's arrays: vectors packed on the
-// device, then everything through two halves of the page-locked staging, one
-// half on the link while host threads empty the other (a pageable copy of whole
-// records and a serial repacking loop took 38 of a 1M-sphere read-back's 40 ms).
+// A getter's device records into the caller's arrays through two halves of the
+// page-locked staging, one half on the link while host threads empty the other
+// (a pageable copy of whole records and a serial repacking loop took 38 of a
+// 1M-sphere read-back's 40 ms).  Vectors are packed by a kernel that writes
+// straight into the staging, so a read-back takes no device memory (a million
+// spheres, 120 MB: 4.0 ms; 4.2 with the vectors packed on the device first and
+// moved by the copy engine).
 class Readback {
   public:
     void vec3(double* host, const double4* src, size_t n) {
@@ -382,70 +384,71 @@ class Readback {
     }
     // Returns the kernels launched; the caller's arrays are filled on return.
     int run(cudaStream_t s) {
-        int launches = 0;
-        size_t words = 0;
-        for (const Item& it : items_)
-            if (it.take3) words += it.bytes / sizeof(double);
-        DBuf<double> packed;
-        packed.alloc(words, s, false);
-        double* q = packed.p;
-        for (Item& it : items_) {
-            if (!it.take3) continue;
-            const size_t n = it.bytes / (3 * sizeof(double));
-            k_take3<<<grid_for(n, 256), 256, 0, s>>>(n, (const double4*)it.src, q);
-            launches++;
-            it.src = (const char*)q;
-            q += 3 * n;
-        }
-        DEMSPH_LAUNCH_CHECK();
+        size_t total = 0;
+        for (const Item& it : items_) total += it.bytes + kAlign;
+        if (items_.empty()) return 0;
         PinnedStage& ps = PinnedStage::get();
         std::lock_guard<std::mutex> lk(ps.m);
-        char* st = ps.reserve(2 * kHalf);
-        if (!st) {  // no page-locked memory: straight into the caller's arrays
-            for (const Item& it : items_)
-                DEMSPH_CUDA(cudaMemcpyAsync(it.host, it.src, it.bytes, cudaMemcpyDeviceToHost, s));
-            DEMSPH_CUDA(cudaStreamSynchronize(s));
-            return launches;
-        }
-        // pieces of at most kHalf bytes, several small items to a half
+        // two halves, or a small one that holds everything
+        const size_t half = total <= kSmall ? kSmall : kHalf;
+        const int halves = total <= kSmall ? 1 : 2;
+        char* st = ps.reserve(halves * half);
+        if (!st) return pageable(s);
+        // whatever ends this call, nothing is still being written when the staging
+        // is unlocked
+        struct Settle {
+            cudaStream_t s;
+            ~Settle() { cudaStreamSynchronize(s); }
+        } settle{s};
+        // pieces of at most `half` bytes, several small items to a half
         struct Half {
             std::vector<Item> part;
             cudaEvent_t ev = nullptr;
             ~Half() {
                 if (ev) cudaEventDestroy(ev);
             }
-        } half[2];
-        for (Half& h : half) DEMSPH_CUDA(cudaEventCreateWithFlags(&h.ev, cudaEventDisableTiming));
+        } part[2];
+        for (Half& h : part) DEMSPH_CUDA(cudaEventCreateWithFlags(&h.ev, cudaEventDisableTiming));
+        int launches = 0;
         size_t k = 0, off = 0;
         auto fill = [&](int h) {
-            half[h].part.clear();
-            size_t used = 0;
-            while (k < items_.size() && used < kHalf) {
+            part[h].part.clear();
+            for (size_t used = 0; k < items_.size() && used < half;) {
                 const Item& it = items_[k];
-                const size_t len = std::min(it.bytes - off, kHalf - used);
-                DEMSPH_CUDA(cudaMemcpyAsync(st + h * kHalf + used, it.src + off, len, cudaMemcpyDeviceToHost, s));
-                half[h].part.push_back({it.host + off, st + h * kHalf + used, len, false});
-                used += len;
+                const size_t len = std::min(it.bytes - off, half - used);
+                char* to = st + h * half + used;
+                if (it.take3) {
+                    const size_t count = len / sizeof(double);
+                    k_take3<<<std::min(grid_for(count, 256), kTakeBlocks), 256, 0, s>>>(
+                        off / sizeof(double), count, (const double*)it.src, (double*)to);
+                    DEMSPH_LAUNCH_CHECK();
+                    launches++;
+                } else {
+                    DEMSPH_CUDA(cudaMemcpyAsync(to, it.src + off, len, cudaMemcpyDeviceToHost, s));
+                }
+                part[h].part.push_back({it.host + off, to, len, false});
+                used += (len + kAlign - 1) / kAlign * kAlign;
                 off += len;
                 if (off == it.bytes) {
                     k++;
                     off = 0;
                 }
             }
-            DEMSPH_CUDA(cudaEventRecord(half[h].ev, s));
+            DEMSPH_CUDA(cudaEventRecord(part[h].ev, s));
         };
         fill(0);
-        for (int h = 0; !half[h].part.empty(); h ^= 1) {
-            fill(h ^ 1);
-            DEMSPH_CUDA(cudaEventSynchronize(half[h].ev));
-            for (const Item& p : half[h].part) host_copy(p.host, p.src, p.bytes);
+        for (int h = 0; !part[h].part.empty(); h ^= 1) {
+            if (halves == 2) fill(h ^ 1);
+            DEMSPH_CUDA(cudaEventSynchronize(part[h].ev));
+            for (const Item& p : part[h].part) host_copy(p.host, p.src, p.bytes);
+            if (halves == 1) break;
         }
-        DEMSPH_CUDA(cudaStreamSynchronize(s));
         return launches;
     }
 
   private:
-    static constexpr size_t kHalf = (size_t)16 << 20;
+    static constexpr size_t kHalf = (size_t)16 << 20, kSmall = (size_t)1 << 20, kAlign = 16;
+    static constexpr unsigned kTakeBlocks = 64;
     struct Item {
         char* host;
         const char* src;
@@ -453,6 +456,33 @@ class Readback {
         bool take3;
     };
     std::vector<Item> items_;
+
+    // No page-locked memory: whole records through a pageable buffer.
+    int pageable(cudaStream_t s) {
+        std::vector<double4> rec;
+        for (const Item& it : items_) {
+            if (!it.take3) {
+                DEMSPH_CUDA(cudaMemcpyAsync(it.host, it.src, it.bytes, cudaMemcpyDeviceToHost, s));
+                continue;
+            }
+            const size_t n = it.bytes / (3 * sizeof(double)), chunk = kHalf / sizeof(double4);
+            rec.resize(std::min(n, chunk));
+            for (size_t i = 0; i < n; i += chunk) {
+                const size_t m = std::min(chunk, n - i);
+                DEMSPH_CUDA(cudaMemcpyAsync(rec.data(), (const double4*)it.src + i, m * sizeof(double4),
+                                            cudaMemcpyDeviceToHost, s));
+                DEMSPH_CUDA(cudaStreamSynchronize(s));
+                double* o = (double*)it.host + 3 * i;
+                for (size_t j = 0; j < m; j++) {
+                    o[3 * j] = rec[j].x;
+                    o[3 * j + 1] = rec[j].y;
+                    o[3 * j + 2] = rec[j].z;
+                }
+            }
+        }
+        DEMSPH_CUDA(cudaStreamSynchronize(s));
+        return 0;
+    }
 };
 
 // Chained launches (programmatic dependent launch): a kernel launched with
