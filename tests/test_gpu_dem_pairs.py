@@ -205,3 +205,25 @@ def test_mixed_contacts_of_like_spheres_keep_their_error(gpu, size, steps, limit
         g.step(steps)
         v[prec] = g.getBall()["velocity"]
     assert rel_err(v["mixed"], v["fp64"]) < limit
+
+
+def test_device_memory_of_a_scene(gpu):
+    """What a scene takes per ball at the default capacities (16 pairs, 16
+    reverse entries, 8 wall candidates): 2,508 B of pair rows and lists, 584 B
+    of wall rows and some 380 B of state and sort (111 of them for a cell of
+    this domain each).  The torques on the pointed balls have no buffer of their
+    own, which would be 512 B."""
+    from .test_zz_no_alloc import _Pool
+
+    n = 200_000
+    pos = np.stack(np.unravel_index(np.arange(n), (59, 59, 59)), 1) * 0.02
+    sc = DEMScene(name="grid", position=pos, radius=np.full(n, 0.005), density=np.full(n, 2500.0),
+                  material=np.zeros(n, np.int32), hertz=[(0, 0, 1e7, 1e7, 0.8, 0.0, 0.0, 0.3, 0.0, 0.0)],
+                  minb=(-0.1,) * 3, maxb=(1.3,) * 3, dt=1e-5)
+    build_dem(sc, "fp64")  # the library's module and pool
+    pool = _Pool()
+    used = pool.attr(pool.USED)
+    g = build_dem(sc, "fp64")
+    per_ball = (pool.attr(pool.USED) - used) / n
+    assert g.capacity()[:2] == (16, 16)
+    assert per_ball < 3600

@@ -1503,7 +1503,7 @@ struct DemScene {
     DBuf<double4> spS[2], spR[2], spT[2];
     int cur = 0;
     bool havePairs = false;
-    DBuf<double4> pF, pTA, pTB;
+    DBuf<double4> pF, pTB;
     DBuf<int> rcnt, rslot;
     DBuf<int4> plist;
     bool pairsStale = false;   // the rows changed outside a rebuild: plist and the reverse lists do not follow them
@@ -1589,7 +1589,9 @@ struct DemScene {
         if (withOld && havePairs) {
             d.pjOld = pj[o].p; d.pcntOld = pcnt[o].p; d.spSOld = spS[o].p; d.spROld = spR[o].p; d.spTOld = spT[o].p;
         }
-        d.pF = pF.p; d.pTA = pTA.p; d.pTB = pTB.p; d.rcnt = rcnt.p; d.rslot = rslot.p; d.plist = plist.p;
+        // (between rebuilds the other half of the sliding springs is free: only the next
+        // rebuild writes it, and what an evaluation puts there it reads itself)
+        d.pF = pF.p; d.pTA = spS[o].p; d.pTB = pTB.p; d.rcnt = rcnt.p; d.rslot = rslot.p; d.plist = plist.p;
         d.accA = 0;
         d.bab = bab.p; d.bok = bok.p; d.bpoint = bpoint.p; d.bnormal = bnormal.p; d.bFs = bFs.p; d.bTb = bTb.p;
         d.bFn = bFn.p; d.bTt = bTt.p; d.bsmax = bsmax.p; d.btmax = btmax.p; d.bF = bF.p; d.bTA = bTA.p; d.bTB = bTB.p;
@@ -1714,7 +1716,6 @@ struct DemScene {
             spT[b].alloc(tors ? n * K : 1, s, true);
         }
         pF.alloc(n * K, s, true);
-        pTA.alloc(n * K, s, true);
         pTB.alloc(n * K, s, true);
         plist.alloc(n * K, s, false);
         rcnt.alloc(n + 1, s, true);
@@ -1745,7 +1746,6 @@ struct DemScene {
                 if (tors) spT[b].grow(n * nk, s);
             }
             pF.alloc(n * nk, s, true);
-            pTA.alloc(n * nk, s, true);
             pTB.alloc(n * nk, s, true);
             plist.alloc(n * nk, s, false);
             K = nk;
