@@ -202,3 +202,23 @@ def test_rows_of_a_large_fluid_overflow_and_are_walked(gpu, prec):
         s.setSPH(position=pos)
         s.step(4)
     _same(a.getSPH(), b.getSPH(), 1e-5)
+
+
+@pytest.mark.parametrize("n,empty", [((24, 24, 26), 1.0), ((25, 24, 25), 1.0), ((25, 24, 25), 2.0), ((25, 24, 25), 3.0)])
+def test_pair_sets_with_plain_and_with_split_cells(gpu, n, empty):
+    """The sort's cells are split along x for fluids of at least 15,000 particles
+    (14,976 and 15,000 here) in domains of no more cells than particles (about
+    2,600, 10,000 and 22,000 here): every pair within the cutoff either way."""
+    sc = _scene(*n)
+    wide = tuple(a + empty * (b - a) if k < 2 else b for k, (a, b) in enumerate(zip(sc.minb, sc.maxb)))
+    g = _build(sc, "mixed", maxb=wide)
+    g.setGraphs(False)
+    g.step(1)
+    x, cut = sc.fluid, 2.0 * 1.3 * sc.spacing
+    key = pair_keys(*g.getPairs(0))
+    from scipy.spatial import cKDTree
+    p = cKDTree(x).query_pairs(cut, output_type="ndarray")
+    d = x[p[:, 0]] - x[p[:, 1]]
+    p = p[(d * d).sum(1) <= cut * cut]
+    both = np.concatenate([p, p[:, ::-1]])
+    np.testing.assert_array_equal(np.sort(key), np.sort(pair_keys(both[:, 0], both[:, 1])))

@@ -2489,8 +2489,9 @@ struct SphScene {
     double listHeadroom = 0.125;  // row capacity above the initial longest row (autotuner)
     CellTable fCells, dCells;
     DBuf<int> fGroups;
-    static constexpr int kFineX = 4;                      // the sort's cells per grid cell along x
-    static constexpr long long kMaxFineCells = 1LL << 25;  // (a larger, mostly empty domain keeps plain cells)
+    static constexpr int kFineX = 4;           // the sort's cells per grid cell along x
+    static constexpr int kFineFluid = 15000;   // smallest fluid that gets them
+    static constexpr int kPartWork = 30000;    // list_parts
     DBuf<double4> pos[2], vel[2], st[2];
     DBuf<double> rho0[2], drho[2];
     DBuf<int> id[2];
@@ -2750,8 +2751,10 @@ struct SphScene {
         constexpr int W = kListShapes[S].warps;
         // a small fluid's cells are fewer than the warps the GPU holds: several
         // warps then share a cell's particles (some twenty), each staging the
-        // cell's candidates for its share.  1,000 particles: 7.8 -> 3.9 us.
-        const int parts = std::min(8, std::max(1, 70000 / std::max(1, N())));
+        // cell's candidates for its share.  1,000 particles: 7.8 -> 3.9 us.  A step
+        // with eight, three and one: 3,456 particles 32.7, 33.3, 34.9 us; 8,192 40.4,
+        // 39.6, 40.0; 16,000 53.0, 51.1, 50.6; 27,648 60.6, 59.2, 56.2.
+        const int parts = std::min(8, std::max(1, kPartWork / std::max(1, N())));
         const int ncoarse = fCells.ncell / fCells.g.rx;
         const unsigned grid = list_grid<S>(std::min(ncoarse, N()) * parts);
         if (withMarkers && nM > 0) {
@@ -3691,8 +3694,12 @@ struct SphScene {
         // Finer cells along x leave a cell's particles in x order: the rows of
         // neighbouring particles then name runs of consecutive particles.  18,000
         // in FP64 73.2 -> 70.0 us a step, eight tanks of a batch 178.8 -> 176.4,
-        // larger fluids within 0.5% (passes 1-2% shorter, list build 8% longer).
-        if ((long long)gd.nx * gd.ny * gd.nz * kFineX <= kMaxFineCells) grid_refine_x(gd, kFineX);
+        // larger fluids within 0.5% (passes 1-2% shorter, list build 8% longer).  Every
+        // cell is counted, scanned and stored, so a small fluid (5,488: 35.4 -> 37.2 us
+        // a step, 11,664: 48.5 -> 51.4; 16,000: 51.6 -> 51.3) and one in a mostly empty
+        // domain (16,000 in 6 million cells 53.9 -> 64.2, 128,000 158.8 -> 170.9) keep
+        // plain cells: a tank has about a quarter of its particles' number of them.
+        if (N() >= kFineFluid && (long long)gd.nx * gd.ny * gd.nz <= N()) grid_refine_x(gd, kFineX);
         status.alloc(1, s, true);
         const int n = N(), nd = ND();
         fCells.setup(gd, n, s);
