@@ -495,10 +495,14 @@ int demsph_sph_snapshot_destroy(demsph_sph_snapshot_t snapshot);
  * density (with the fluid's h) runs momentum and continuity passes
  * specialised for it (constants hoisted, terms regrouped; same pairs, same
  * formulas), coupled scenes included (the markers' terms as in the general
- * passes); enable = 0 keeps the general passes.  uniform_kernels reports
- * whether the specialised passes are in use. */
+ * passes).  An FP64 scene of that kind without coupled bodies, whose
+ * smoothing length and densities lie between 1e-9 and 1e9, runs such passes in
+ * double precision.  enable = 0 keeps the general passes in either precision.
+ * uniform_kernels reports whether the specialised mixed-precision passes are in
+ * use, uniform_kernels_fp64 whether the FP64 ones are. */
 int demsph_sph_set_uniform_kernels(demsph_sph_t s, int enable);
 int demsph_sph_uniform_kernels(demsph_sph_t s, int* active);
+int demsph_sph_uniform_kernels_fp64(demsph_sph_t s, int* active);
 /* No counterpart in the reference.  FP64 conservation diagnostics of the
  * fluid, summed on the device in a fixed order, 8 doubles: mass, momentum
  * (3), kinetic energy, potential energy -sum m g.x, sum of the density

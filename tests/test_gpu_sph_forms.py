@@ -222,3 +222,19 @@ def test_pair_sets_with_plain_and_with_split_cells(gpu, n, empty):
     p = p[(d * d).sum(1) <= cut * cut]
     both = np.concatenate([p, p[:, ::-1]])
     np.testing.assert_array_equal(np.sort(key), np.sort(pair_keys(both[:, 0], both[:, 1])))
+
+
+def test_which_scenes_run_the_fp64_passes(gpu):
+    """Uniform constants, lengths and densities inside the range of the FP32
+    approximations their reciprocals start from, and no coupled bodies."""
+    for n in ((4, 4, 4), (21, 20, 20)):
+        assert _build(_scene(*n), "fp64").uniformKernelsFP64() and _build(_scene(*n), "mixed").uniformKernels()
+        assert not _build(_scene(*n), "mixed").uniformKernelsFP64()
+        assert not _build(_scene(*n), "fp64", uniform=False).uniformKernelsFP64()
+    light = _scene(4, 4, 4)
+    light.density = 1e-10
+    assert not _build(light, "fp64").uniformKernelsFP64()
+    sc = scenes.balls_in_tank(nx=10, ny=10, depth=10, balls=((0.5, 0.5, 0.5, 2.0, 1200.0),))
+    f, d, c = scenes.build_coupled(sc, "fp64")
+    c.step(1, sc.dem_substeps)
+    assert not f.uniformKernelsFP64()

@@ -68,6 +68,7 @@ SIGNATURES = {
     "demsph_sph_restore": [_vp, _vp],
     "demsph_sph_snapshot_destroy": [_vp],
     "demsph_sph_uniform_kernels": [_vp, _i],
+    "demsph_sph_uniform_kernels_fp64": [_vp, _i],
     "launchAddConstantForce": [_vp, _vp, _sz, _sz, _sz, _vp],
     "launchAddGlobalDampingForceTorque": [_vp, _vp, _vp, _vp, _dbl, _sz, _sz, _sz, _vp],
     "launchAddBuoyancyDrag": [_vp, _vp, _vp, _vp, _vp, _dbl, _dbl, Double3, Double3, _dbl, _sz, _sz, _sz, _vp],

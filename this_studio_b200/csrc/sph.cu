@@ -4231,6 +4231,14 @@ int demsph_sph_uniform_kernels(demsph_sph_t h, int* active) {
         *active = h->sc.ready && h->sc.uni_path() ? 1 : 0;
     });
 }
+int demsph_sph_uniform_kernels_fp64(demsph_sph_t h, int* active) {
+    return guarded([&] {
+        SPH_CHECK(h);
+        if (!active) throw Status(DEMSPH_ERR_INVALID, "null output pointer");
+        h->sc.sync_mode();
+        *active = h->sc.ready && h->sc.uni64_path() ? 1 : 0;
+    });
+}
 struct demsph_sph_snapshot {
     demsph_sph_t scene = nullptr;
     SphScene::Snap snap;

@@ -585,13 +585,19 @@ class WCSPHSolver:
 
     def setUniformKernels(self, enable=True):
         """Use (default) or not the passes specialised for uniform particle
-        constants (mixed precision)."""
+        constants."""
         call("demsph_sph_set_uniform_kernels", self._h, int(bool(enable)))
 
     def uniformKernels(self):
         """Whether the specialised mixed-precision passes are in use."""
         a = C.c_int()
         call("demsph_sph_uniform_kernels", self._h, C.byref(a))
+        return bool(a.value)
+
+    def uniformKernelsFP64(self):
+        """Whether the specialised FP64 passes are in use."""
+        a = C.c_int()
+        call("demsph_sph_uniform_kernels_fp64", self._h, C.byref(a))
         return bool(a.value)
 
     def diagnostics(self):
