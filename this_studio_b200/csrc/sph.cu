@@ -1883,10 +1883,13 @@ __device__ __forceinline__ void skin_pairs(int cnt, const int* __restrict__ nbV,
 // Resident blocks.  First pass: 61 us at 7 blocks, 64 at 8 (128,000), 438 and
 // 431 (a million); 9 and 10 spill in its loops (5% and 26% longer than 8).  The
 // second fits 9 (a million: 296 us at 8, 280 at 9, 296 at 10).
-template <bool kSkin, bool kMarkers>
-constexpr int kUniAccelBlocks = kMarkers || kSkin ? 8 : 9;
+// Sixteen lanes a particle: seven blocks per SM hold the largest fluid that runs
+// so, without the spills of eight (5,488: 35.2 -> 34.4 us a step; at six 8,192 take
+// 41.7 instead of 37.3).
+template <bool kSkin, bool kMarkers, int kLanes>
+constexpr int kUniAccelBlocks = kLanes != kQuad ? 7 : kMarkers || kSkin ? 8 : 9;
 template <bool kSkin, bool kMarkers = false, int kLanes = kQuad>
-__global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers>)
+__global__ void __launch_bounds__(kSphBlock, kUniAccelBlocks<kSkin, kMarkers, kLanes>)
     k_sph_accel_u(SphDev d, double hdt, double dt, int first) {
     const int i = uni_particle<kLanes>();
     if (i >= d.N) return;
