@@ -38,8 +38,10 @@ the data path); value = all ranks' particle-steps / max-over-ranks time.
 from __future__ import annotations
 
 import argparse
+import hashlib
 import json
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -359,6 +361,30 @@ def served_stream(torch, num, seed=5, rate=100.0, steps=500, chunk=100, fp64_sam
             "per_kind": m["per_kind"], "per_kind_vs_plain": kinds, "autotune": tune}
 
 
+CAPTURED_SOURCES = ("this_studio_b200/csrc/sph.cu", "this_studio_b200/csrc/common.cuh")
+
+
+def code_hash(path):
+    """sha256 of a CUDA source without its comments and white space."""
+    text = open(path).read()
+    text = re.sub(r"/\*.*?\*/", " ", text, flags=re.S)
+    text = re.sub(r"//[^\n]*", " ", text)
+    return hashlib.sha256(re.sub(r"\s+", "", text).encode()).hexdigest()
+
+
+def captured_counts(path=None, root=ROOT):
+    """profiles/traffic.json, the bytes, instructions and flop per launch of the
+    committed ncu capture; {} when the kernels' code has changed since (counts
+    of other kernels over the time of these would be no measurement)."""
+    path = path or os.path.join(root, "profiles", "traffic.json")
+    if not os.path.exists(path):
+        return {}
+    tj = json.load(open(path))
+    same = tj.get("code_sha256", {})
+    ok = all(same.get(p) == code_hash(os.path.join(root, p)) for p in CAPTURED_SOURCES)
+    return tj if ok else {}
+
+
 def pipeline_traffic(tj):
     """DRAM bytes per launch of the momentum kernel inside the step (caches as
     the step leaves them, L2 flushed between steps): first and second pass
@@ -432,10 +458,7 @@ def native(args, rank, world, dist):
     for a, b in zip(sc.minb, sc.maxb):
         ncell *= max(1, int((b - a) / (2.0 * 1.3 * sc.spacing * 1.04)))
     step_bytes = sph_bytes_8d(nf, nd, ncell)
-    tj = {}
-    tpath = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(tpath):
-        tj = json.load(open(tpath))
+    tj = captured_counts()
     traffic = tj.get("k_sph_accel_bytes_per_launch")
     inst = tj.get("k_sph_accel_warp_instructions_per_launch")
     flop = tj.get("k_sph_accel_fp32_flop_per_launch")
@@ -529,11 +552,12 @@ def native(args, rank, world, dist):
         # the bounds the SPH passes actually sit at: FP32 SIMT throughput and
         # warp-instruction issue (4 per SM per clock; 148 SMs at the sampled
         # SM clock); flop and instruction counts per launch from the committed
-        # ncu capture, time live
+        # ncu capture (null when the kernels have changed since), time live
         "fp32_simt": None if not flop else {
             "kernel": "k_sph_accel_u", "achieved": flop / (mom_ms / 1e3) / 1e12, "unit": "TFLOP/s",
             "peak": fp32_peak / 1e12, "frac": flop / (mom_ms / 1e3) / fp32_peak, "flop_per_launch": flop,
-            "source": "profiles/traffic.json (ncu: 2 x ffma + fadd + fmul thread instructions)"},
+            "source": "profiles/traffic.json (ncu thread instructions: 4 x ffma2 + 2 x (fadd2 + fmul2 + ffma) + "
+                      "fadd + fmul)"},
         "issue_roofline": None if not inst else {
             "kernel": "k_sph_accel_u", "achieved": inst / (mom_ms / 1e3), "unit": "warp-instructions/s",
             "peak": 4 * 148 * sm_hz, "frac": inst / (mom_ms / 1e3) / (4 * 148 * sm_hz),

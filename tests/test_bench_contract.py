@@ -48,3 +48,27 @@ def test_reference_arm_under_torchrun():
     lines = _lines(r.stdout)
     assert len(lines) == 1
     _check(lines[0], 2)
+
+
+def test_counts_of_other_kernels_are_not_reported(tmp_path):
+    """The captured counts belong to the code they were captured from: a change
+    of the kernels drops them, one of their comments does not."""
+    sys.path.insert(0, ROOT)
+    import bench
+
+    for p in bench.CAPTURED_SOURCES:
+        (tmp_path / p).parent.mkdir(parents=True, exist_ok=True)
+        (tmp_path / p).write_text("// one\n__global__ void k(int* a) { /* two */ a[0] = 1; }\n")
+    (tmp_path / "profiles").mkdir()
+    js = tmp_path / "profiles" / "traffic.json"
+    assert bench.captured_counts(root=str(tmp_path)) == {}
+    sha = {p: bench.code_hash(str(tmp_path / p)) for p in bench.CAPTURED_SOURCES}
+    js.write_text(json.dumps({"k_sph_accel_bytes_per_launch": 5, "code_sha256": sha}))
+    assert bench.captured_counts(root=str(tmp_path))["k_sph_accel_bytes_per_launch"] == 5
+    src = tmp_path / bench.CAPTURED_SOURCES[0]
+    src.write_text("__global__ void k(int* a)\n{ a[0] = 1;  // three\n}\n")
+    assert bench.captured_counts(root=str(tmp_path))["k_sph_accel_bytes_per_launch"] == 5
+    src.write_text("__global__ void k(int* a) { a[0] = 2; }")
+    assert bench.captured_counts(root=str(tmp_path)) == {}
+    js.write_text(json.dumps({"k_sph_accel_bytes_per_launch": 5}))
+    assert bench.captured_counts(root=str(tmp_path)) == {}
