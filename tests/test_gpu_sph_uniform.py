@@ -83,7 +83,7 @@ def test_uniform_trajectory_and_pairs(gpu, oracle_lib, dam):
 
 def test_uniform_passes_with_markers(gpu, oracle_lib):
     """A coupled scene (uniform fluid and dummy constants, markers on three
-    balls) runs the specialised passes with unpacked shadows: 20 coupled
+    balls) runs the specialised passes: 20 coupled
     steps give the same ball forces, fluid and ball trajectories as the
     general passes within the FP32 rounding of the regrouped terms, and both
     stay within the 1e-5 target of the FP64 oracle."""

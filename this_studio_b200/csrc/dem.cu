@@ -177,10 +177,10 @@ __device__ __forceinline__ void record_pair(const DemDev& d, int slot, int A, in
 // order.  kLanes = 1: one thread per ball with the next row's bounds loaded
 // ahead and four candidates in flight.  Candidates are read as the sort's
 // cell-ordered FP32 records; a ball's own record is fetched only for a pair in
-// the test's uncertain band (RECORD_FIGURES).  Against a candidate-by-candidate walk: 4,096
-// touching spheres 40.7 -> 11.5 us (eight lanes; one lane with its loads
-// unrolled took 24.5), 64,000 36.0 -> 26.1 us, 10^6 falling spheres 108 -> 94 us
-// (eight lanes there: 343).
+// the test's uncertain band.  Against a candidate-by-candidate walk of the FP64
+// records: 4,096 touching spheres 40.7 -> 10.1 us (eight lanes; one lane with its
+// loads unrolled took 24.5), 64,000 36.0 -> 25.2 us, 10^6 falling spheres
+// 108 -> 84 us (eight lanes there: 343).
 template <int kLanes>
 __global__ void __launch_bounds__(128, kLanes == 1 ? 6 : 8) k_dem_build_pairs(DemDev d) {
     const int t = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
@@ -1539,9 +1539,13 @@ struct DemScene {
     // 4,096-sphere bounce 23.4 -> 21.4 us per step in FP64, 19.9 -> 19.6
     // mixed, the touching pack 53.9 -> 52.5; the 220k beam was 0.8% slower.
     static constexpr int kChainBalls = 65536;
-    static constexpr int kBuildLaneBalls = 16384;  // up to this size eight lanes build a ball's row
-    // Up to this size four lanes finish a ball (a beam of 110,000: 22.5 us on
-    // four, 14.5 on one; a pack of 64,000 the same either way).
+    // Up to this size eight lanes build a ball's row (a step of 13,824 touching
+    // spheres 25.6 us with eight and 26.9 with one, of 21,952 28.4 and 28.8, of
+    // 32,768 35.5 and 34.9).
+    static constexpr int kBuildLaneBalls = 16384;
+    // Up to this size four lanes finish a ball (a step of 21,952 touching spheres
+    // 28.8 us with four and 29.7 with one, of 46,656 43.3 and 41.6; 29,791 falling
+    // ones 16.9 and 16.0; the finish of a beam of 110,000 22.5 and 14.5).
     static constexpr int kLaneBalls = 32768;
 
     // Periodic boundaries (setPeriodicBoundary, DEMSolver.h:1944-1959): one

@@ -615,7 +615,8 @@ __global__ void k_sph_permute(int n, const int* __restrict__ sorted, const doubl
 
 // countSPHInteractionsKernel / writeSPHInteractionsKernel and the dummy pair
 // kernels (SPHNeighborSearchKernel.cu:6-228) in one pass: j != i,
-// |r_ij| <= 2 max(h_i, h_j), rows in the reference's stencil order.
+// |r_ij| <= 2 max(h_i, h_j), rows in the order of the stencil's cells (the
+// reference's within cells that are not split; getPairs sorts them by its keys).
 //
 // Built one warp per cell that holds fluid -- per group of the finer cells the
 // particles are sorted by, which make up a cell; the reorder lists the groups,
@@ -1598,10 +1599,11 @@ __global__ void __launch_bounds__(kSphBlock, kDensityBlocks<R>) k_sph_density(Sp
 //               - (rho_i + rho_j) (v_j - v_i) . r'] / (2 rho_j (rho_i + rho_j)).
 // A lane takes its neighbours two at a time in packed FP32 (add / mul / fma
 // .f32x2: one issue for both).  A dam
-// break of 128,000 against one neighbour at a time: first pass 64.7 -> 63.5 us,
-// second 46.2 -> 38.6, continuity 45.4 -> 40.5; of a million 424 -> 431,
-// 327 -> 270, 315 -> 277.  What is left waits for the gathers (7 of 13 stalled
-// warps, L1 at 62% of its data wavefronts, 42% of the issue slots).
+// break of 128,000 against one neighbour at a time: first pass 64.7 -> 61.7 us,
+// second 46.2 -> 40.3, continuity 45.4 -> 40.7; of a million 424 -> 415,
+// 327 -> 277, 315 -> 277.  What is left waits for the gathers (5.5 to 9.9 stalled
+// warps an issue, L1 at 55 to 61% of its data wavefronts, 44 to 58% of the issue
+// slots).
 // The fluid shadows are packed (k_sph_pack): the fixed-point position
 // carries rho in w and the FP32 velocity carries p, so a fluid neighbour is
 // two 16-byte gathers (the general passes gather a third record, the FP32
@@ -1630,10 +1632,12 @@ __device__ __forceinline__ float2 nrcp2(float2 x) {
 // not fill the GPU and which waits for a quad's chain of some twenty
 // neighbours, four quads that take every fourth pair of row entries.
 // 1,000 particles: first pass, second and continuity 18.0, 10.9
-// and 10.8 us on quads, one neighbour at a time, 7.1, 4.4 and 4.5 so; 18,000 in
-// FP64 were slower (79.9 us a step against 74.7).
+// and 10.8 us on quads, one neighbour at a time, 6.9, 4.1 and 4.4 so.
 constexpr int kWide = 16;
-constexpr int kWideFluid = 8192;  // largest fluid that runs on kWide lanes per particle
+// Largest fluid that runs on kWide lanes per particle.  A step on sixteen lanes and
+// on quads: 8,192 particles 40 and 50 us (FP64 54 and 58), 11,664 49 and 51 (60
+// and 61), 16,000 54 and 51 (70 and 65).
+constexpr int kWideFluid = 8192;
 template <int kLanes>
 __device__ __forceinline__ int uni_particle() {
     return (int)(blockIdx.x * (kSphBlock / kLanes) + threadIdx.x / kLanes);
@@ -1880,9 +1884,9 @@ __device__ __forceinline__ void skin_pairs(int cnt, const int* __restrict__ nbV,
     if (lig == 0) cntOut[i] = over ? -1 : (kLaneRows | lanes);
 }
 
-// Resident blocks.  First pass: 61 us at 7 blocks, 64 at 8 (128,000), 438 and
-// 431 (a million); 9 and 10 spill in its loops (5% and 26% longer than 8).  The
-// second fits 9 (a million: 296 us at 8, 280 at 9, 296 at 10).
+// Resident blocks.  First pass at 7, 8 and 9: 59.7, 58.7 and 61.0 us at 128,000
+// (fresh lists), 410, 388 and 403 at a million, with markers 60.3, 58.8 and 61.9
+// (a tank of 110,000).  Second at 8, 9 and 10: 37.3, 39.4 and 47.5; 273, 264 and 335.
 // Sixteen lanes a particle: seven blocks per SM hold the largest fluid that runs
 // so, without the spills of eight (5,488: 35.2 -> 34.4 us a step; at six 8,192 take
 // 41.7 instead of 37.3).
@@ -2047,15 +2051,15 @@ __global__ void __launch_bounds__(kSphBlock, 8) k_sph_density_u(SphDev d, double
 
 // ---------------------------------------------------------------------------
 // FP64 passes for scenes with uniform particle constants and no markers: the
-// regrouped terms above in double precision, one neighbour at a time.  The
+// regrouped terms above in double precision, two neighbours side by side.  The
 // general FP64 passes are bound by the FP64 pipe and by their gathers (three
 // 32-byte records per fluid neighbour, four divisions or square roots per
 // pair); here a neighbour is two records (xr, vp), each one 32-byte load, and
 // a pair takes one reciprocal square root and one reciprocal.  128,000: first
-// pass 162 -> 95 us, second 127 -> 73, continuity 126 -> 68.  Side by side two
-// neighbours hold more registers: a fluid whose blocks all fit the GPU at four
-// per SM runs so (18,000: 20, 15 and 14 us; 74.7 -> 69.9 us a step), a larger
-// one at six (at four 311 us a step against 295).
+// pass 162 -> 95 us, second 127 -> 72, continuity 126 -> 70.  A fluid whose blocks
+// all fit the GPU at four per SM runs with the registers of four (18,000: 19, 15
+// and 14 us; 74.7 -> 69.9 us a step), a larger one with those of six (at four 311
+// us a step against 295).
 //
 // 1 / sqrt(x) and 1 / x from the FP32 approximation y0 (relative error below
 // 2^-21) by one step of Halley's respectively the cubic Newton-Schulz series in
@@ -2268,8 +2272,8 @@ template <class R>
 constexpr int kMarkerForceBlocks = std::is_same<R, float>::value ? 8 : 4;
 // kPacked: the fluid's shadows are packed (the specialised passes'), its h, m, c
 // and nu the scene's constants; unpacked, the passes themselves gathered a third
-// record per neighbour (coupled tank of 190,000: first pass 93.2 -> 88.5 us,
-// second 73.8 -> 67.6, continuity 77.6 -> 65.0; the reaction is unchanged).
+// record per neighbour (coupled tank of 190,000: second pass 73.8 -> 68.0 us,
+// continuity 77.6 -> 65.3; the reaction is unchanged).
 template <class R, bool kSkinRows, bool kPacked = false>
 __global__ void __launch_bounds__(kSphBlock, kMarkerForceBlocks<R>) k_sph_marker_force(SphDev d, double w, int add) {
     const int t = blockIdx.x * kSphPerBlock + threadIdx.x / kQuad;
@@ -2494,7 +2498,7 @@ struct SphScene {
     DBuf<int> fGroups;
     static constexpr int kFineX = 4;           // the sort's cells per grid cell along x
     static constexpr int kFineFluid = 15000;   // smallest fluid that gets them
-    static constexpr int kPartWork = 30000;    // list_parts
+    static constexpr int kPartWork = 30000;    // particles over which one warp takes a whole list cell
     DBuf<double4> pos[2], vel[2], st[2];
     DBuf<double> rho0[2], drho[2];
     DBuf<int> id[2];
