@@ -55,9 +55,9 @@ def test_read_back_takes_no_device_memory(gpu):
     s.initialize((-0.1,) * 3, (1.3,) * 3, (0, 0, -9.81), 1e-5)
     g = build_dem(scenes.bonded_beam_clumps(nx=30, ny=5, nz=5, n_clumps=40), "fp64")
     pool = _Pool()
-    pool.reset_high()
     used = pool.attr(pool.USED)
+    pool.reset_high()
     np.testing.assert_array_equal(s.getBall()["position"], pos)
     g.getBondedInteraction()
     g.getClump()
-    assert pool.attr(pool.USED) == used and pool.attr(pool.USED_HIGH) == used
+    assert pool.attr(pool.USED_HIGH) <= used  # (other scenes' memory may be given back meanwhile)
